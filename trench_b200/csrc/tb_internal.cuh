@@ -42,9 +42,10 @@ __host__ __device__ __forceinline__ int tb_pad_row(int pj, int ny) {
 // corners (pi, pj), (pi+1, pj), (pi, pj+1), (pi+1, pj+1) -- has four vacuum cells.
 // A step of less than half a cell that starts inside such a quad ends in one of its
 // corner cells, so it cannot reach a wall, and its vacuum weights sum to one.
-// Quads beyond the last corner column or row (never a particle's quad) report false.
+// Quads beyond the last corner column or row (never a particle's quad) report false, and so
+// do the quads of the top and bottom halo rows, where a step may leave the grid.
 __device__ __forceinline__ bool tb_quad_vacuum(const uint8_t *vac, int nx, int ny, int pi, int pj) {
-    if (pi > nx || pj > ny) return false;
+    if (pi > nx || pj >= ny || pj == 0) return false;
     const int c0 = tb_pad_col(pi, nx) * ny, c1 = tb_pad_col(pi + 1, nx) * ny;
     const int r0 = tb_pad_row(pj, ny), r1 = tb_pad_row(pj + 1, ny);
     return vac[c0 + r0] && vac[c0 + r1] && vac[c1 + r0] && vac[c1 + r1];

@@ -4,16 +4,22 @@
 // roots are the hardware approximations (max 2 ulp), denormals flush to zero (the
 // vacuum flag stored in the low bit of a zero field is such a denormal).
 // Design (B200-first):
-//  * Position = integer cell + FP32 offset in [0,1) cell units, so the cell
-//    index, periodic wrap and floor are exact integer operations and the offset
-//    keeps 2^-24-cell resolution everywhere in the grid.
+//  * Position = nearest grid vertex (integers) + FP32 offset in [-0.5, 0.5] cells, so the
+//    index and the periodic wrap are exact integer operations, the offset keeps 2^-25-cell
+//    resolution everywhere in the grid, and the vertex is the index of the bilinear quad.
 //  * Velocities in units of vscale (m/s); time in dx/vscale; the packed field is
 //    E*vac*dx/vscale^2 so qm*field is the acceleration in these units.
 //  * The packed field (8 bytes per cell, vacuum flag in bit 0 of Ex) is staged
 //    once per block into shared memory with a bulk async copy (TMA engine,
-//    cp.async.bulk + mbarrier); every bilinear gather is a shared-memory load.
+//    cp.async.bulk + mbarrier); every bilinear gather is a shared-memory load.  A lane
+//    keeps its quad's corners in registers and loads only when it changes quad.
 //    Grids too large for shared memory read the same layout from global memory
 //    (L2-resident).
+//  * Three forms of a step.  While every active lane of a warp is in an open quad (no
+//    solid corner, not at the top or bottom edge) the warp runs step_open, which has no
+//    branch; with any lane near a wall it runs step_near, whose extra arithmetic is
+//    branch-free too; a step that meets a wall, a corner or the edge is not taken there but
+//    left to step_decide, which runs for several such lanes at once.
 //  * Persistent warps, one particle per lane, lanes refill from a global atomic
 //    queue as soon as their particle ends (no lane waits for a slow electron); a warp
 //    reserves a small block of ranks at a time and prefetches their particles into
@@ -22,10 +28,15 @@
 //    then ions longest predicted first from per-bin step means of the previous trace,
 //    claimed through FP32 claim records written in that order by a scatter kernel.
 //  * Absorbed particles are deposited with integer atomics (bit-exact counts).
-//  * The x/y-symmetric arithmetic of a step (half-cell shift, the bilinear sums of
-//    (Ex, Ey), acceleration, velocity and position updates, cell remainder) runs on
-//    packed FP32 pairs (sm_100 f32x2 add/mul/fma): one instruction per pair, which
-//    cuts the issued instructions of this issue-bound loop by about an eighth.
+//  * The x/y-symmetric arithmetic of a step (the bilinear sums of (Ex, Ey), acceleration,
+//    velocity and position updates, rounding to the vertex) runs on packed FP32 pairs
+//    (sm_100 f32x2 add/mul/fma): one instruction per pair.
+// What bounds it: instruction issue.  Open space (an all-vacuum 60 x 200 grid, 2.4M
+// particles): 69.9 warp instructions and 80 cycles per scheduler and warp-step, 87 % of the
+// issue slots (before the vertex frame, the cached quads and the three forms: 87.9
+// instructions, 107 cycles; without the cached quads the gathers' bank conflicts, 24 shared-
+// memory wavefronts a warp-step, held it at 102).  AR-8 trench, 2^20 particles: 1.257 ms
+// against 1.416 ms a launch; walls are near some lane in 45 % of the warp-steps.
 // The step follows the reference algorithm (trench_charging_2d.py:584-650,
 // trench_trace.cu:92-148): vacuum-weighted bilinear field, CFL step, trapezoid
 // update, periodic x, escape at the top, staircase corner crossing, first-face
@@ -38,7 +49,6 @@
 namespace {
 
 constexpr int F32_THREADS = 1024;
-constexpr float ONE_BELOW = 0x1.fffffep-1f;  // largest float < 1
 
 struct K32 {
     tb_trace_args a;
@@ -72,8 +82,7 @@ struct K32 {
     const float4 *rf_barrier;
     const float4 *rf_wave;          // (vs_i, vm_i, vs_i+1 - vs_i, vm_i+1 - vm_i), i < n_phase
     float t_clock;                  // clock units (2^-32 period) per unit of step time
-    float wave_scale;               // n_phase * 2^-32: clock -> table position
-    int n_phase_m1;
+    bool short_steps;               // every step is under half a period (clock steps fit 32 bits)
     float t_sec;                    // seconds per unit of step time (dx / vscale)
     float dt_max;                   // step bound of the in-flight field, in step time
     float bvs, bvm;                 // largest voltage deltas of the waveform
@@ -81,7 +90,7 @@ struct K32 {
 
 // 1.0f for a vacuum cell, 0.0f for a solid one, with integer operations only
 __device__ __forceinline__ float vac_of(const tb_fcell &c) {
-    return __uint_as_float((__float_as_uint(c.ex) & 1u) ? 0x3f800000u : 0u);
+    return __uint_as_float((__float_as_uint(c.ex) & 1u) * 0x3f800000u);
 }
 
 template <bool SMEM>
@@ -91,6 +100,9 @@ struct FieldView {
         if (SMEM) return p[c];
         const float2 v = __ldg(reinterpret_cast<const float2 *>(p) + c);
         return tb_fcell{v.x, v.y};
+    }
+    __device__ __forceinline__ uint32_t shared_address() const {
+        return static_cast<uint32_t>(__cvta_generic_to_shared(p));
     }
     __device__ __forceinline__ bool vac(int c) const {
         float x;
@@ -135,22 +147,86 @@ __device__ bool stage_field(void *dst, const void *src, int bytes, uint64_t *mba
     return __syncthreads_and(done) != 0;
 }
 
-// One lane's particle: cell (ix, iy) and FP32 offset (ox, oy) in [0,1) cell units,
-// velocity in vscale units; pid < 0 = no particle.
+// One lane's particle.  The position is held relative to the nearest grid vertex: vertex
+// (cx, cy) is the corner shared by padded cells (cx, cy) .. (cx + 1, cy + 1), so it is also the
+// index of the bilinear quad the particle interpolates from, and u in [-0.5, 0.5] is the offset
+// from it in cells (two bits finer than an offset in [0, 1), and tx = u + 0.5 needs no selects).
+// cx in [0, nx] (0 and nx are the same vertex), cy in [0, ny]; a particle below the grid (open
+// bottom rows only) has cy = 0 and the rest of its distance in u.y.  Velocity in vscale units;
+// hq is half the charge-to-mass ratio.  pid < 0 = no particle.
 struct LaneState {
-    int pid, ix, iy, steps, stop_at, spc;
-    float2 o, v;                    // offset (ox, oy) and velocity (vx, vy), packed pairs
-    float qm;
+    int pid, cx, cy, steps, stop_at, spc;
+    float2 u, v;                    // offset and velocity, packed pairs
+    float hq;
     uint32_t clock;                 // circuit_rf: clock in 2^-32 of the period
     float elapsed;                  // circuit_rf: seconds in flight
 };
 
-// The four bilinear corners a lane loaded last and their base index (-1 = none).  With
-// the field in global memory a step that stays in the same cell quad reuses them: a
-// move is under half a cell at the usual CFL, so about half the steps skip the gathers.
+// Adding MAGIC (1.5 x 2^23) to a value below 2^22 rounds it to the nearest integer, which the
+// low mantissa bits then hold: as_int(x + MAGIC) - MAGIC_BITS.  Nearest-vertex indices come
+// from this instead of floor and float-to-int conversions (both on the conversion pipe, at a
+// quarter of the packed-add rate).
+constexpr float MAGIC = 12582912.f;
+constexpr int MAGIC_BITS = 0x4b400000;
+
+// Vertex and offset of a coordinate in cells, clamped into a grid of n cells; the row keeps
+// the distance below the grid in the offset (see LaneState).
+__device__ __forceinline__ void vertex_of(double xc, int cell, int *c, float *u) {
+    const double d = fmin(fmax(xc - (double)cell, 0.0), 1.0 - 0x1p-24);
+    const int h = d >= 0.5 ? 1 : 0;
+    *c = cell + h;
+    *u = (float)(d - (double)h);
+}
+__device__ __forceinline__ void start_position(const double x, const double y, double inv_dx, int nx, int ny, int *cx,
+                                               int *cy, float2 *u) {
+    // x lies in cell min(int(x/dx), nx-1) as in the reference (trench_charging_2d.py:611); a
+    // start above the grid escapes at once
+    const double xc = x * inv_dx, yc = y * inv_dx;
+    vertex_of(xc, min(max((int)xc, 0), nx - 1), cx, &u->x);
+    if (yc < 0.0) {
+        *cy = 0;
+        u->y = (float)fmax(yc, -1e6);
+    } else {
+        vertex_of(yc, min((int)yc, ny - 1), cy, &u->y);
+    }
+}
+
+// The four bilinear corners of a lane's quad and their base index (-1 = none).  A step
+// moves under half a cell at the usual CFL, so about half the steps stay in the quad and
+// reload nothing: fewer lanes per gather means fewer shared-memory bank conflicts (or L1
+// lines).  The corners of the next quad are loaded at the end of a step, ahead of the
+// loop's vote.
 struct QuadCache {
     int base;
     tb_fcell c00, c01, c10, c11;
+    // an inactive lane's quad, so that it does not hold its warp up; load() after base = -1 undoes it
+    __device__ __forceinline__ void mark_open() { c00.ey = __uint_as_float(__float_as_uint(c00.ey) | 1u); }
+    // `last`: the largest base whose four corners lie in the field (a particle with a field
+    // or velocity that is not finite may hold any index)
+    template <bool SMEM>
+    __device__ __forceinline__ void load(const FieldView<SMEM> &F, int at, int P, int last) {
+        const int b = (int)min((unsigned)at, (unsigned)last);
+        if (SMEM) {
+            // predicated in place: a branch around the loads costs more than the loads
+            const uint32_t a0 = F.shared_address() + 8u * (unsigned)b, a1 = a0 + 8u * (unsigned)P;
+            asm volatile(
+                "{\n\t.reg .pred c;\n\t"
+                "setp.ne.s32 c, %8, %9;\n\t"
+                "@c ld.shared.v2.f32 {%0, %1}, [%10];\n\t"
+                "@c ld.shared.v2.f32 {%2, %3}, [%10 + 8];\n\t"
+                "@c ld.shared.v2.f32 {%4, %5}, [%11];\n\t"
+                "@c ld.shared.v2.f32 {%6, %7}, [%11 + 8];\n\t}"
+                : "+f"(c00.ex), "+f"(c00.ey), "+f"(c01.ex), "+f"(c01.ey), "+f"(c10.ex), "+f"(c10.ey), "+f"(c11.ex),
+                  "+f"(c11.ey)
+                : "r"(b), "r"(base), "r"(a0), "r"(a1)
+                : "memory");
+            base = b;
+        } else if (b != base) {
+            c00 = F.at(b); c01 = F.at(b + 1);
+            c10 = F.at(b + P); c11 = F.at(b + P + 1);
+            base = b;
+        }
+    }
 };
 
 // Per-lane event counts, reduced over the warp at the end.
@@ -158,28 +234,29 @@ struct LaneTally {
     unsigned steps, esc_i, esc_e, lost, hit_i, hit_e;
 };
 
+// The quad flag of a quad's lower-left corner: all four cells vacuum, and no step leaves the grid.
+__device__ __forceinline__ bool is_open(const tb_fcell &c00) { return __float_as_uint(c00.ey) & 1u; }
+
 // Loop-invariant parameters of one case.
 template <bool SMEM>
 struct CaseView {
     FieldView<SMEM> F;
     int nx, ny, cells, P;
+    int last;           // largest quad index
     float inv_v, cfl;
     bool barrier, tapered, first_face;
     bool small_steps;   // cfl < 1/2: a step ends in a corner cell of its start quad
 };
 
-// One step of one particle (trench_charging_2d.py:584-650): vacuum-weighted bilinear
-// field, CFL step, trapezoid update, periodic x, escape, staircase corner, first-face
-// wall entry and barrier reflection; on absorption, escape or the step cap the
-// particle's outputs are written and s.pid becomes -1.
-// Waveform table position of a clock: interval i and the position within it
-// (trench_rf.py:5-11: periodic linear interpolation of n_phase samples; the last
-// interval runs to the first sample).
+// Waveform table position of a clock: interval i and the position w within it in [0, 1)
+// (trench_rf.py:5-11: periodic linear interpolation of n_phase samples; the last interval
+// runs to the first sample).  The clock is a 32-bit fraction of the period, so clock x
+// n_phase is the table position as a 32.32 fixed-point number: the high word is the
+// interval, the top 23 bits of the low word are the mantissa of 1 + w.
 __device__ __forceinline__ int rf_interval(const K32 &k, uint32_t clock, float &w) {
-    const float f = (float)clock * k.wave_scale;
-    const int i = min((int)f, k.n_phase_m1);  // a clock just below 2^32 may round up to n
-    w = f - (float)i;
-    return i;
+    const unsigned long long f = (unsigned long long)clock * (unsigned)k.a.n_phase;
+    w = __uint_as_float(0x3f800000u | ((uint32_t)f >> 9)) - 1.f;
+    return (int)(f >> 32);
 }
 
 // Voltage deltas (substrate, mask) of the waveform at a clock.
@@ -190,187 +267,307 @@ __device__ __forceinline__ void rf_voltages(const K32 &k, uint32_t clock, float 
     vm = fmaf(w, e.w, e.y);
 }
 
-template <bool SMEM, bool RF>
-__device__ __forceinline__ void step_particle(const K32 &k, const CaseView<SMEM> &C, LaneState &s, LaneTally &t,
-                                              QuadCache &q) {
-    const tb_trace_args &a = k.a;
-    const int nx = C.nx, ny = C.ny, P = C.P;
-    // ---- vacuum-weighted bilinear field (trench_charging_2d.py:492-509) ----
-    // corners (i0, j0) = (ix - 1 + hx, iy - 1 + hy) .. (i0 + 1, j0 + 1); in the halo-padded
-    // field i0 + 1 = ix + hx needs no wrap and the clipped rows need one clamp
-    const int hx = s.o.x >= 0.5f ? 1 : 0, hy = s.o.y >= 0.5f ? 1 : 0;
-    const float2 tq = __fadd2_rn(s.o, make_float2(hx ? -0.5f : 0.5f, hy ? -0.5f : 0.5f));
-    const float tx = tq.x, ty = tq.y;
-    const int base = (s.ix + hx) * P + max(s.iy + hy, 0);
-    tb_fcell c00, c01, c10, c11;
-    if (SMEM) {
-        c00 = C.F.at(base); c01 = C.F.at(base + 1);
-        c10 = C.F.at(base + P); c11 = C.F.at(base + P + 1);
-    } else {
-        if (base != q.base) {
-            q.c00 = C.F.at(base); q.c01 = C.F.at(base + 1);
-            q.c10 = C.F.at(base + P); q.c11 = C.F.at(base + P + 1);
-            q.base = base;
-        }
-        c00 = q.c00; c01 = q.c01; c10 = q.c10; c11 = q.c11;
-    }
-    // A step moves at most cfl cells (|v| dt + |a| dt^2 / 2 <= cfl for the CFL dt), so with
-    // cfl below one half a step that starts inside this quad of cell centres ends in one of
-    // its four corner cells.  The quad flag (bit 0 of the lower-left corner's ey) says all
-    // four are vacuum: then the step cannot reach a wall and the vacuum weights sum to one,
-    // and both the normalisation and the end-cell checks are skipped.
-    const bool near = !(C.small_steps && (__float_as_uint(c00.ey) & 1u));
-    // bilinear sum of the (vacuum-premultiplied) field with (ex, ey) as one packed pair:
-    // along y in both columns, then along x
+// Bilinear sum of a packed pair over a quad's corners: along y in both columns, then along x.
+__device__ __forceinline__ float2 bilinear2(float2 f00, float2 f01, float2 f10, float2 f11, float2 tx, float2 ty) {
     const float2 M1 = make_float2(-1.f, -1.f);
-    const float2 tyy = make_float2(ty, ty), txx = make_float2(tx, tx);
-    const float2 f00 = make_float2(c00.ex, c00.ey), f01 = make_float2(c01.ex, c01.ey);
-    const float2 f10 = make_float2(c10.ex, c10.ey), f11 = make_float2(c11.ex, c11.ey);
-    const float2 e0 = __ffma2_rn(tyy, __ffma2_rn(f00, M1, f01), f00);
-    const float2 e1 = __ffma2_rn(tyy, __ffma2_rn(f10, M1, f11), f10);
-    const float2 E = __ffma2_rn(txx, __ffma2_rn(e0, M1, e1), e0);
-    const float sex = E.x, sey = E.y;
-    float inv_sw = 1.f;
-    if (near) {
+    const float2 e0 = __ffma2_rn(ty, __ffma2_rn(f00, M1, f01), f00);
+    const float2 e1 = __ffma2_rn(ty, __ffma2_rn(f10, M1, f11), f10);
+    return __ffma2_rn(tx, __ffma2_rn(e0, M1, e1), e0);
+}
+
+// Column position of a particle in [0, nx) cells.
+__device__ __forceinline__ double wrap_column(double x, int nx) {
+    return x < 0.0 ? x + nx : (x >= nx ? x - nx : x);
+}
+
+// Writes the outputs of a particle that is absorbed (1), escaped (2) or stopped at its step
+// cap (3) and empties the lane.
+template <bool RF>
+__device__ __forceinline__ void finish_particle(const K32 &k, LaneState &s, LaneTally &t, int done) {
+    const tb_trace_args &a = k.a;
+    const int pid = s.pid;
+    t.steps += (unsigned)s.steps;   // the claim subtracted the particle's earlier steps
+    a.d_steps[pid] = s.steps;
+    if (done == 3) {
+        if (s.steps >= a.max_steps) ++t.lost;
+    } else {
+        a.d_status[pid] = (int8_t)done;
+    }
+    if (done == 3 || a.write_state) {
+        a.d_x[pid] = wrap_column((double)s.cx + (double)s.u.x, k.nx) * k.dx;
+        a.d_y[pid] = ((double)s.cy + (double)s.u.y) * k.dx;
+        a.d_vx[pid] = (double)s.v.x * k.vscale;
+        a.d_vy[pid] = (double)s.v.y * k.vscale;
+    }
+    if (RF) {
+        a.d_clock[2 * pid] = (double)s.clock * 0x1p-32 * a.period;
+        a.d_clock[2 * pid + 1] = (double)s.elapsed;
+    }
+    s.pid = -1;
+}
+
+// Half acceleration h, time step and (circuit_rf) clock advance of a particle's next step
+// (trench_charging_2d.py:492-509, 587-608): vacuum-weighted bilinear field and the CFL step
+// dt = cfl / (|v| + sqrt(2 |a|) + 1 m/s), with sqrt(2 |a|) = 2 (|h|^2)^(1/4).  NEAR: the quad may
+// hold solid corners, whose weights are left out; otherwise the vacuum weights sum to one.
+template <bool SMEM, bool RF, bool NEAR>
+__device__ __forceinline__ void step_size(const K32 &k, const CaseView<SMEM> &C, const LaneState &s,
+                                          const QuadCache &q, float2 &h, float &dt, uint32_t &inc) {
+    const float tx = s.u.x + 0.5f, ty = s.u.y + 0.5f;
+    const float2 txx = make_float2(tx, tx), tyy = make_float2(ty, ty);
+    const tb_fcell c00 = q.c00, c01 = q.c01, c10 = q.c10, c11 = q.c11;
+    float2 E = bilinear2(make_float2(c00.ex, c00.ey), make_float2(c01.ex, c01.ey), make_float2(c10.ex, c10.ey),
+                         make_float2(c11.ex, c11.ey), txx, tyy);
+    float hqs = s.hq;
+    if (NEAR) {
+        // no branch: some lane of the warp needs it, and an open quad's own value is selected
         const float v00 = vac_of(c00), v01 = vac_of(c01), v10 = vac_of(c10), v11 = vac_of(c11);
         const float s0 = fmaf(ty, v01 - v00, v00), s1 = fmaf(ty, v11 - v10, v10);
-        inv_sw = __fdividef(1.f, fmaxf(fmaf(tx, s1 - s0, s0), 1e-12f));
+        const float hqn = __fdividef(hqs, fmaxf(fmaf(tx, s1 - s0, s0), 1e-12f));
+        hqs = is_open(c00) ? hqs : hqn;
     }
-    float2 A;
-    float dt;
-    const float speed = sqrtf(fmaf(s.v.x, s.v.x, s.v.y * s.v.y));
+    const float speed = sqrtf(fmaf(s.v.x, s.v.x, s.v.y * s.v.y)) + C.inv_v;
+    inc = 0u;
     if (!RF) {
-        const float qs = s.qm * inv_sw;
-        A = __fmul2_rn(make_float2(qs, qs), E);
-        const float acc = sqrtf(fmaf(A.x, A.x, A.y * A.y));
-        dt = __fdividef(C.cfl, speed + sqrtf(2.f * acc) + C.inv_v);
+        h = __fmul2_rn(make_float2(hqs, hqs), E);
+        dt = __fdividef(C.cfl, fmaf(2.f, sqrtf(sqrtf(fmaf(h.x, h.x, h.y * h.y))), speed));
     } else {
-        const float ux = 1.f - tx, uy = 1.f - ty;
-        const float w00 = ux * uy, w10 = tx * uy, w01 = ux * ty, w11 = tx * ty;
         // in-flight RF field (trench_trace.cu:97-110): the basis fields at the same corners
         // and weights bound the step, and the field is taken at the mid-step clock.  The
         // waveform interval of the start clock is loaded before the step is known: a
         // CFL-limited step is far shorter than an interval, so the mid-step clock is
         // nearly always in it and the lookup leaves the step's dependency chain.
         const uint32_t c0 = s.clock;
+        const int base = q.base, P = C.P;
         float w0;
         const int i0 = rf_interval(k, c0, w0);
         const float4 e0 = __ldg(k.rf_wave + i0);
         const float4 b00 = __ldg(k.rf_field + base), b01 = __ldg(k.rf_field + base + 1);
         const float4 b10 = __ldg(k.rf_field + base + P), b11 = __ldg(k.rf_field + base + P + 1);
-        // weighted sums like the field's; the vacuum normalisation 1/sw is applied once
-        const float sxs = w00 * b00.x + w10 * b10.x + w01 * b01.x + w11 * b11.x;
-        const float sys = w00 * b00.y + w10 * b10.y + w01 * b01.y + w11 * b11.y;
-        const float sxm = w00 * b00.z + w10 * b10.z + w01 * b01.z + w11 * b11.z;
-        const float sym = w00 * b00.w + w10 * b10.w + w01 * b01.w + w11 * b11.w;
-        const float bx = fabsf(sex) + (k.bvs * fabsf(sxs) + k.bvm * fabsf(sxm));
-        const float by = fabsf(sey) + (k.bvs * fabsf(sys) + k.bvm * fabsf(sym));
-        const float accel = fabsf(s.qm) * inv_sw * sqrtf(bx * bx + by * by);
-        dt = fminf(k.dt_max, __fdividef(C.cfl, speed + sqrtf(2.f * accel) + C.inv_v));
-        const unsigned long long inc = __float2ull_rn(dt * k.t_clock);
-        const uint32_t mid = c0 + (uint32_t)(inc >> 1);
+        const float2 Es = bilinear2(make_float2(b00.x, b00.y), make_float2(b01.x, b01.y), make_float2(b10.x, b10.y),
+                                    make_float2(b11.x, b11.y), txx, tyy);
+        const float2 Em = bilinear2(make_float2(b00.z, b00.w), make_float2(b01.z, b01.w), make_float2(b10.z, b10.w),
+                                    make_float2(b11.z, b11.w), txx, tyy);
+        const float bx = hqs * (fabsf(E.x) + fmaf(k.bvs, fabsf(Es.x), k.bvm * fabsf(Em.x)));
+        const float by = hqs * (fabsf(E.y) + fmaf(k.bvs, fabsf(Es.y), k.bvm * fabsf(Em.y)));
+        dt = fminf(k.dt_max, __fdividef(C.cfl, fmaf(2.f, sqrtf(sqrtf(fmaf(bx, bx, by * by))), speed)));
+        // clock advance in 2^-32 of the period; a step bound below the period fits 32 bits
+        uint32_t mid;
+        if (k.short_steps) {
+            inc = __float2uint_rn(dt * k.t_clock);
+            mid = c0 + (inc >> 1);
+        } else {
+            const unsigned long long w64 = __float2ull_rn(dt * k.t_clock);
+            inc = (uint32_t)w64;
+            mid = c0 + (uint32_t)(w64 >> 1);
+        }
         float w;
         const int im = rf_interval(k, mid, w);
         const float4 e = im == i0 ? e0 : __ldg(k.rf_wave + im);
         const float vs = fmaf(w, e.z, e.x), vm = fmaf(w, e.w, e.y);
-        const float qs = s.qm * inv_sw;
-        A = make_float2(qs * (sex + (vs * sxs + vm * sxm)), qs * (sey + (vs * sys + vm * sym)));
-        s.clock = c0 + (uint32_t)inc;
+        E = __ffma2_rn(make_float2(vs, vs), Es, E);
+        E = __ffma2_rn(make_float2(vm, vm), Em, E);
+        h = __fmul2_rn(make_float2(hqs, hqs), E);
+    }
+}
+
+// New offset from the present vertex, x + v dt + h dt^2, in (-1.5, 1.5).
+__device__ __forceinline__ float2 moved(const LaneState &s, float2 h, float dt) {
+    const float dd = dt * dt;
+    return __ffma2_rn(h, make_float2(dd, dd), __ffma2_rn(s.v, make_float2(dt, dt), s.u));
+}
+// Its nearest integers (the vertex change) as rounded sums, see MAGIC, and the remainders (exact).
+__device__ __forceinline__ float2 rounded(float2 p) { return __fadd2_rn(p, make_float2(MAGIC, MAGIC)); }
+__device__ __forceinline__ float2 remainder2(float2 p, float2 r) {
+    return __ffma2_rn(__fadd2_rn(r, make_float2(-MAGIC, -MAGIC)), make_float2(-1.f, -1.f), p);
+}
+__device__ __forceinline__ int vertex_change(float r) { return __float_as_int(r) - MAGIC_BITS; }
+// periodic x: vertices -1 and nx + 1 wrap (as unsigned, the wrapped index is the smaller)
+__device__ __forceinline__ int wrap_vertex(int c, int nx) {
+    const unsigned a = __viaddmin_u32((unsigned)c, (unsigned)nx, (unsigned)c);
+    return (int)__viaddmin_u32(a, (unsigned)-nx, a);
+}
+
+// Takes a step of length dt to offset p (r = rounded(p)) from the present vertex.
+template <bool SMEM, bool RF>
+__device__ __forceinline__ void take_step(const K32 &k, const CaseView<SMEM> &C, LaneState &s, QuadCache &q, float2 h,
+                                          float dt, uint32_t inc, float2 p, float2 r) {
+    const float d2 = dt + dt;
+    s.cx = wrap_vertex(s.cx + vertex_change(r.x), C.nx);
+    s.cy += vertex_change(r.y);
+    s.v = __ffma2_rn(h, make_float2(d2, d2), s.v);
+    s.u = remainder2(p, r);
+    if (RF) {
+        s.clock += inc;
         s.elapsed += dt * k.t_sec;
     }
+    q.load(C.F, s.cx * C.P + s.cy, C.P, C.last);
+}
 
-    // ---- CFL step and trapezoid update (trench_charging_2d.py:587-608) ----
-    // v' = v + a dt and the move (v + v') dt / 2 = (v + a dt / 2) dt, each a packed pair.
-    // A step moves less than one cell, so the new offset lies in (-1, 2): the cell change
-    // is its floor (-1, 0 or 1) and the new offset the remainder (exact for the shift by
-    // 1; a remainder that rounds up to 1 is clamped below 1)
-    const float2 dtt = make_float2(dt, dt);
-    const float hdt = 0.5f * dt;
-    const float2 vn = __ffma2_rn(A, dtt, s.v);
-    const float2 S = __fmul2_rn(__ffma2_rn(A, make_float2(hdt, hdt), s.v), dtt);
-    const float vxn = vn.x, vyn = vn.y, sx = S.x, sy = S.y;
-    const float2 pos = __fadd2_rn(s.o, S);
-    const float fnx = floorf(pos.x), fny = floorf(pos.y);
-    const int dix = (int)fnx, diy = (int)fny;
-    const float2 rem = __ffma2_rn(make_float2(fnx, fny), M1, pos);
-    const float nox = fminf(rem.x, ONE_BELOW), noy = fminf(rem.y, ONE_BELOW);
-    int nix = s.ix + dix;
-    nix = nix < 0 ? nx - 1 : (nix >= nx ? 0 : nix);
-    const int niy = s.iy + diy;
-    ++s.steps;
-    const bool escaped = niy >= ny;
-    bool hit_end = false, corner = false;
+// A step of a warp whose lanes' quads are all open: a step moves at most cfl cells (|v| dt +
+// |a| dt^2 / 2 <= cfl for the CFL dt), so with cfl below one half it ends in one of the quad's
+// four corner cells, all vacuum.  Inactive lanes take a step of length zero, which leaves them
+// exactly as they are.
+template <bool SMEM, bool RF>
+__device__ __forceinline__ void step_open(const K32 &k, const CaseView<SMEM> &C, LaneState &s, QuadCache &q,
+                                          bool active) {
+    float2 h;
+    float dt;
+    uint32_t inc;
+    step_size<SMEM, RF, false>(k, C, s, q, h, dt, inc);
+    if (!active) {
+        dt = 0.f;
+        inc = 0u;
+    }
+    const float2 p = moved(s, h, dt);
+    take_step<SMEM, RF>(k, C, s, q, h, dt, inc, p, rounded(p));
+}
+
+// A step of a warp with lanes near a wall or an edge of the grid.  It is taken if it ends in a
+// vacuum cell of the grid with no staircase corner on the way; otherwise the particle stays as
+// it was and the return is false: the step needs the decisions of step_decide.
+template <bool SMEM, bool RF>
+__device__ __forceinline__ bool step_near(const K32 &k, const CaseView<SMEM> &C, LaneState &s, QuadCache &q,
+                                          bool active) {
+    float2 h;
+    float dt;
+    uint32_t inc;
+    step_size<SMEM, RF, true>(k, C, s, q, h, dt, inc);
+    float2 p = moved(s, h, dt), r = rounded(p);
+    bool go;
+    if (C.small_steps) {
+        // the end cell is the corner of the quad on the side of the offset's signs
+        const int px = __float_as_int(p.x), py = __float_as_int(p.y);
+        const float f = px < 0 ? (py < 0 ? q.c00.ex : q.c01.ex) : (py < 0 ? q.c10.ex : q.c11.ex);
+        const bool diagonal = C.tapered && ((px ^ __float_as_int(s.u.x)) & (py ^ __float_as_int(s.u.y))) < 0;
+        go = is_open(q.c00) ||
+             ((__float_as_uint(f) & 1u) && (unsigned)(s.cy + (py >> 31)) < (unsigned)C.ny && !diagonal);
+    } else {
+        const float2 un = remainder2(p, r);
+        // padded cell of the end and of the start (a move that is not finite ends nowhere)
+        const int cxw = wrap_vertex(s.cx + vertex_change(r.x), C.nx), cyn = s.cy + vertex_change(r.y);
+        const int ec = cxw + 1 + (__float_as_int(un.x) >> 31), er = cyn + 1 + (__float_as_int(un.y) >> 31);
+        const int sc = s.cx + 1 + (__float_as_int(s.u.x) >> 31), sr = s.cy + 1 + (__float_as_int(s.u.y) >> 31);
+        go = (unsigned)cxw <= (unsigned)C.nx && (unsigned)(er - 1) < (unsigned)C.ny && cyn >= 0 &&
+             C.F.vac(ec * C.P + er) && !(C.tapered && ec != sc && er != sr);
+    }
+    go = go && active;
+    if (!go) {
+        dt = 0.f;
+        inc = 0u;
+        p = s.u;
+        r = make_float2(MAGIC, MAGIC);
+    }
+    take_step<SMEM, RF>(k, C, s, q, h, dt, inc, p, r);
+    return go;
+}
+
+// One step of one particle with everything it may meet (trench_charging_2d.py:584-650):
+// escape, staircase corner, first-face wall entry, barrier reflection, the step cap (s.steps
+// counts the step already); an ended particle's outputs are written and s.pid becomes -1.
+template <bool SMEM, bool RF>
+__device__ __forceinline__ void step_decide(const K32 &k, const CaseView<SMEM> &C, LaneState &s, LaneTally &t,
+                                            QuadCache &q) {
+    const int nx = C.nx, ny = C.ny, P = C.P;
+    float2 h;
+    float dt;
+    uint32_t inc;
+    step_size<SMEM, RF, true>(k, C, s, q, h, dt, inc);
+    const bool near = !(C.small_steps && is_open(q.c00));
+    const float2 p = moved(s, h, dt), r = rounded(p);
+    const float dd = dt * dt, d2 = dt + dt;
+    const float2 vn = __ffma2_rn(h, make_float2(d2, d2), s.v);
+    float2 un = remainder2(p, r);
+    const int cxn = s.cx + vertex_change(r.x);
+    int cyn = s.cy + vertex_change(r.y);
+    int cxw = wrap_vertex(cxn, nx);
+    const tb_trace_args &a = k.a;
+    const float2 move = __ffma2_rn(h, make_float2(dd, dd), __fmul2_rn(s.v, make_float2(dt, dt)));
+    int dix = cxn - s.cx;
+    if (!(fabsf(p.x) < 2.f && fabsf(p.y) < 4e6f)) {
+        // not a finite move: the particle stays where it is until its step cap
+        cxw = s.cx; cyn = s.cy; un = s.u;
+        dix = 0;
+    }
+    cxw = min(max(cxw, 0), nx);   // a one-column grid can step past the wrap
+    if (cyn < 0) {
+        un.y += (float)cyn;
+        cyn = 0;
+    }
+    // padded cell (column, row) of the start and of the end, rows clipped like the
+    // reference; the column and row changes between them
+    const int sx = s.u.x >= 0.f ? 1 : 0, ex = un.x >= 0.f ? 1 : 0;
+    const int sr = min(max(s.cy + (s.u.y >= 0.f ? 1 : 0), 1), ny);
+    const int sc = s.cx + sx, ec = cxw + ex;
+    const int er0 = cyn + (un.y >= 0.f ? 1 : 0);
+    const bool escaped = er0 > ny;
+    const int er = min(max(er0, 1), ny);
+    dix += ex - sx;
+    const int diy = er - sr;
+    bool hit = false, corner = false, x_first = false, reflected = false;
     if (near && !escaped) {
-        hit_end = !C.F.vac((nix + 1) * P + max(niy, -1) + 1);
-        // both the column and the (clipped) row changed: a staircase corner may lie on
-        // the path between two vacuum cells (trench_charging_2d.py:614-621).  The move
-        // reaches the wall only if the cell beyond the first boundary crossed is solid
-        // (the first-face rule of the rare path below, same expressions), so that is
-        // decided here and the rare path runs only for an actual corner contact.
-        corner = C.tapered && !hit_end && dix != 0 && max(niy, 0) != max(s.iy, 0);
-        if (corner) {
-            const int y0c = min(max(s.iy, 0), ny - 1);
-            const int iyn = min(max(niy, 0), ny - 1);
-            const float fx = ((dix > 0 ? 1.f : 0.f) - s.o.x) / sx;
-            const float fy = ((iyn > y0c ? 1.f : 0.f) - s.o.y) / sy;
-            const bool x_first = fx < fy;
-            corner = !C.F.vac((x_first ? nix + 1 : s.ix + 1) * P + (x_first ? y0c : iyn) + 1);
-        }
+        hit = !C.F.vac(ec * P + er);
+        // both the column and the row changed: a staircase corner may lie on the path
+        // between two vacuum cells (trench_charging_2d.py:614-621)
+        corner = C.tapered && !hit && dix != 0 && diy != 0;
     }
-
-    if (!(hit_end || corner || escaped || s.steps >= s.stop_at)) {
-        s.ix = nix; s.iy = niy; s.o = make_float2(nox, noy); s.v = vn;
-        return;
-    }
-
-    // ---- rare path: wall contact, escape, or step cap ----
-    const int y0c = min(max(s.iy, 0), ny - 1);
-    const int iyn = min(max(niy, 0), ny - 1);
-    const int diy_e = iyn - y0c;     // rows clipped like the reference
-    bool hit = hit_end;
-    int dcell = nix * ny + iyn;
-    bool reflected = false;
+    int hc = ec, hr = er;            // padded cell of the deposit
     if (hit ? C.first_face : corner) {
         // first solid face crossed (trench_charging_2d.py:512-539) in cell units
         const float inf = __int_as_float(0x7f800000);
-        const float fx = dix != 0 ? ((dix > 0 ? 1.f : 0.f) - s.o.x) / sx : inf;
-        const float fy = diy_e != 0 ? ((diy_e > 0 ? 1.f : 0.f) - s.o.y) / sy : inf;
-        const bool x_first = fx < fy;
-        const int ax_ = x_first ? nix : s.ix, ay_ = x_first ? y0c : y0c + diy_e;
-        const bool use_last = dix != 0 && diy_e != 0 && C.F.vac((ax_ + 1) * P + ay_ + 1);
-        const int cx = use_last ? nix : ax_, cy = use_last ? y0c + diy_e : ay_;
+        const float fx = dix != 0 ? ((float)(sx - 1 + (dix > 0 ? 1 : 0)) - s.u.x) / move.x : inf;
+        const float fy = diy != 0 ? ((float)(sr - 1 - s.cy + (diy > 0 ? 1 : 0)) - s.u.y) / move.y : inf;
+        x_first = fx < fy;
+        const int ac = x_first ? ec : sc, ar = x_first ? sr : er;
+        const bool use_last = dix != 0 && diy != 0 && C.F.vac(ac * P + ar);
+        hc = use_last ? ec : ac;
+        hr = use_last ? er : ar;
         const bool face_x = use_last ? !x_first : x_first;
-        const int ccell = cx * ny + cy;
-        hit = !C.F.vac((cx + 1) * P + cy + 1);
-        dcell = ccell;
+        hit = !C.F.vac(hc * P + hr);
         if (hit && C.barrier) {
+            const int ccell = (hc == 0 ? nx - 1 : hc > nx ? 0 : hc - 1) * ny + hr - 1;
             const float4 b = __ldg(k.barrier + ccell);
             // neighbour the particle came from: W/E across an x face, S/N across a y face
-            float dphi = face_x ? (dix > 0 ? b.x : b.y) : (diy_e > 0 ? b.z : b.w);
+            float dphi = face_x ? (dix > 0 ? b.x : b.y) : (diy > 0 ? b.z : b.w);
             if (RF) {
                 // barrier of the instantaneous potential at the clock after the step
                 // (trench_trace.cu:131-136)
                 float vs, vm;
-                rf_voltages(k, s.clock, vs, vm);
+                rf_voltages(k, s.clock + inc, vs, vm);
                 const float4 bs = __ldg(k.rf_barrier + ccell), bm = __ldg(k.rf_barrier + C.cells + ccell);
-                const float ds = face_x ? (dix > 0 ? bs.x : bs.y) : (diy_e > 0 ? bs.z : bs.w);
-                const float dm = face_x ? (dix > 0 ? bm.x : bm.y) : (diy_e > 0 ? bm.z : bm.w);
+                const float ds = face_x ? (dix > 0 ? bs.x : bs.y) : (diy > 0 ? bs.z : bs.w);
+                const float dm = face_x ? (dix > 0 ? bm.x : bm.y) : (diy > 0 ? bm.z : bm.w);
                 dphi += vs * ds + vm * dm;
             }
-            const float vn = face_x ? vxn : vyn;
-            if (0.5f * vn * vn < s.qm * dphi) {
+            const float vnorm = face_x ? vn.x : vn.y;
+            if (0.25f * vnorm * vnorm < s.hq * dphi) {
                 // reflect: the normal velocity flips, the position stays at the start point
-                s.v.x = face_x ? -vxn : vxn;
-                s.v.y = face_x ? vyn : -vyn;
+                s.v.x = face_x ? -vn.x : vn.x;
+                s.v.y = face_x ? vn.y : -vn.y;
+                if (RF) {
+                    s.clock += inc;
+                    s.elapsed += dt * k.t_sec;
+                }
                 hit = false;
                 reflected = true;
             }
         }
     }
-    if (!reflected) { s.ix = nix; s.iy = niy; s.o = make_float2(nox, noy); s.v = vn; }
+    if (!reflected) {
+        if (escaped) {              // the quad index stays in the grid
+            un.y += (float)(cyn - ny);
+            cyn = ny;
+        }
+        s.cx = cxw; s.cy = cyn; s.u = un; s.v = vn;
+        if (RF) {
+            s.clock += inc;
+            s.elapsed += dt * k.t_sec;
+        }
+        q.load(C.F, cxw * P + cyn, P, C.last);
+    }
 
-    int done = 0;
     if (hit) {
+        const int dcell = (hc == 0 ? nx - 1 : hc > nx ? 0 : hc - 1) * ny + hr - 1;
         if (dcell < 0 || dcell >= C.cells) {
             atomicCAS(k.err, TB_DERR_NONE, TB_DERR_BAD_CELL);
         } else {
@@ -378,54 +575,33 @@ __device__ __forceinline__ void step_particle(const K32 &k, const CaseView<SMEM>
         }
         if (a.d_hit) a.d_hit[s.pid] = dcell;
         if (s.spc == 0) ++t.hit_i; else ++t.hit_e;
-        done = 1;
+        finish_particle<RF>(k, s, t, 1);
     } else if (escaped && !reflected) {
         if (s.spc == 0) ++t.esc_i; else ++t.esc_e;
-        done = 2;
+        finish_particle<RF>(k, s, t, 2);
     } else if (s.steps >= s.stop_at) {
-        if (s.steps >= a.max_steps) ++t.lost;
-        done = 3;
-    }
-    if (done) {
-        const int pid = s.pid;
-        t.steps += (unsigned)s.steps;   // the claim subtracted the particle's earlier steps
-        a.d_steps[pid] = s.steps;
-        if (done != 3) a.d_status[pid] = (int8_t)done;
-        if (done == 3 || a.write_state) {
-            a.d_x[pid] = ((double)s.ix + (double)s.o.x) * k.dx;
-            a.d_y[pid] = ((double)s.iy + (double)s.o.y) * k.dx;
-            a.d_vx[pid] = (double)s.v.x * k.vscale;
-            a.d_vy[pid] = (double)s.v.y * k.vscale;
-        }
-        if (RF) {
-            a.d_clock[2 * pid] = (double)s.clock * 0x1p-32 * a.period;
-            a.d_clock[2 * pid + 1] = (double)s.elapsed;
-        }
-        s.pid = -1;
+        finish_particle<RF>(k, s, t, 3);
     }
 }
 
 // Shared-memory pool of particle states for the drain of a case: 9 words per lane
-// (struct of arrays over the block's threads): pid; ix | iy << 16 (grids below 32768
-// cells a side, iy >= -1); steps; stop_at | spc << 31; ox, oy, vx, vy, qm.
+// (struct of arrays over the block's threads): pid; cx | cy << 16 (grids below 32767
+// cells a side); steps; stop_at | spc << 31; ux, uy, vx, vy, hq.
 constexpr int POOL_WORDS = 9;
 constexpr int POOL_WORDS_RF = 11;   // + phase, elapsed
-#ifndef TB_TAIL_ROUND_STEPS
-#define TB_TAIL_ROUND_STEPS 64
-#endif
-constexpr int TAIL_ROUND_STEPS = TB_TAIL_ROUND_STEPS;
+constexpr int TAIL_ROUND_STEPS = 64;
 
 template <bool RF>
 __device__ __forceinline__ void pool_put(uint32_t *P, int T, int q, const LaneState &s) {
     P[0 * T + q] = (uint32_t)s.pid;
-    P[1 * T + q] = ((uint32_t)s.ix & 0xffffu) | ((uint32_t)s.iy << 16);
+    P[1 * T + q] = (uint32_t)s.cx | ((uint32_t)s.cy << 16);
     P[2 * T + q] = (uint32_t)s.steps;
     P[3 * T + q] = (uint32_t)s.stop_at | ((uint32_t)s.spc << 31);
-    P[4 * T + q] = __float_as_uint(s.o.x);
-    P[5 * T + q] = __float_as_uint(s.o.y);
+    P[4 * T + q] = __float_as_uint(s.u.x);
+    P[5 * T + q] = __float_as_uint(s.u.y);
     P[6 * T + q] = __float_as_uint(s.v.x);
     P[7 * T + q] = __float_as_uint(s.v.y);
-    P[8 * T + q] = __float_as_uint(s.qm);
+    P[8 * T + q] = __float_as_uint(s.hq);
     if (RF) {
         P[9 * T + q] = s.clock;
         P[10 * T + q] = __float_as_uint(s.elapsed);
@@ -436,30 +612,93 @@ template <bool RF>
 __device__ __forceinline__ void pool_get(const uint32_t *P, int T, int q, LaneState &s) {
     s.pid = (int)P[0 * T + q];
     const uint32_t xy = P[1 * T + q];
-    s.ix = (int)(xy & 0xffffu);
-    s.iy = (int)xy >> 16;  // arithmetic shift keeps iy = -1
+    s.cx = (int)(xy & 0xffffu);
+    s.cy = (int)(xy >> 16);
     s.steps = (int)P[2 * T + q];
     const uint32_t w = P[3 * T + q];
     s.stop_at = (int)(w & 0x7fffffffu);
     s.spc = (int)(w >> 31);
-    s.o.x = __uint_as_float(P[4 * T + q]);
-    s.o.y = __uint_as_float(P[5 * T + q]);
+    s.u.x = __uint_as_float(P[4 * T + q]);
+    s.u.y = __uint_as_float(P[5 * T + q]);
     s.v.x = __uint_as_float(P[6 * T + q]);
     s.v.y = __uint_as_float(P[7 * T + q]);
-    s.qm = __uint_as_float(P[8 * T + q]);
+    s.hq = __uint_as_float(P[8 * T + q]);
     if (RF) {
         s.clock = P[9 * T + q];
         s.elapsed = __uint_as_float(P[10 * T + q]);
     }
 }
 
+// Steps the warp's active lanes together until fewer than `least` are left (a lane whose step
+// needs a decision does not take it and goes inactive), or the first reaches its step cap, or
+// after `limit` steps; particles at their cap end here.  Returns the steps made.  Every lane
+// of the warp calls it.  While every active lane's quad is open the whole warp runs step_open,
+// which has no branch; the cached quad of an inactive lane is marked open.
+template <bool SMEM, bool RF>
+__device__ __forceinline__ int step_warp(const K32 &k, const CaseView<SMEM> &C, LaneState &s, LaneTally &t,
+                                         QuadCache &q, bool &active, int limit, int least) {
+    const unsigned FULL = 0xffffffffu;
+    const int n = (int)min((unsigned)limit, __reduce_min_sync(FULL, active ? (unsigned)(s.stop_at - s.steps)
+                                                                           : 0x7fffffffu));
+    int j = 0;
+    for (;;) {
+        if (C.small_steps && __all_sync(FULL, is_open(q.c00))) {
+            step_open<SMEM, RF>(k, C, s, q, active);
+            if (++j >= n) break;
+        } else {
+            if (!step_near<SMEM, RF>(k, C, s, q, active) && active) {
+                s.steps += j;
+                active = false;
+                q.mark_open();
+            }
+            if (++j >= n || __popc(__ballot_sync(FULL, active)) < least) break;
+        }
+    }
+    if (active) {
+        s.steps += j;
+        if (s.steps >= s.stop_at) {
+            finish_particle<RF>(k, s, t, 3);
+            active = false;
+            q.mark_open();
+        }
+    }
+    return j;
+}
+
+// The decision steps of the held lanes (occupied, not active).
+template <bool SMEM, bool RF>
+__device__ __forceinline__ void step_held(const K32 &k, const CaseView<SMEM> &C, LaneState &s, LaneTally &t,
+                                          QuadCache &q, bool &active) {
+    if (s.pid >= 0 && !active) {
+        s.cx = min(max(s.cx, 0), C.nx);   // any index after steps that were not finite
+        s.cy = min(s.cy, C.ny);
+        if (s.cy < 0) {                   // below the grid (see LaneState)
+            s.u.y += (float)s.cy;
+            s.cy = 0;
+        }
+        q.base = -1;
+        q.load(C.F, s.cx * C.P + s.cy, C.P, C.last);
+        ++s.steps;
+        step_decide<SMEM, RF>(k, C, s, t, q);
+        active = s.pid >= 0;
+        if (!active) q.mark_open();
+    }
+}
+
+// Lanes that wait, held for a decision step or empty, before the warp runs the decision
+// steps and the refill for all of them.  Both are long, rarely taken code (about 280
+// instructions) that would otherwise run for one lane at a time; a waiting lane costs a
+// thirty-second of the warp.  2, 3, 4, 6 lanes: 1549, 1473, 1441, 1426 us a batch (AR-8, 2^20
+// particles), 4240, 3974, 3847, 3758 us (2^22 particles, untapered).
+constexpr int WAIT_LANES = 6;
+
 // Traces particles of one case with the calling block until the case's queue is
 // drained and every particle has ended, then adds the warps' tallies to the case's
 // totals.  `fieldp` is the packed field in shared or global memory.  Every thread of
 // the block calls it.
 //
-// Main phase: each lane takes a particle from the case's global queue whenever its
-// particle ends.  Drain: once the queue is empty a warp keeps only the lanes whose
+// Main phase: each lane takes a particle from the case's global queue when its
+// particle has ended.  Drain: once the queue is empty a warp keeps only the lanes whose
 // particles are still in flight, so with independent warps the block would issue
 // nearly full instruction streams for a few live lanes each until the longest
 // particle ends.  With a shared-memory pool (pool != nullptr) the block instead runs
@@ -479,6 +718,7 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
     C.ny = k.ny;
     C.cells = k.nx * k.ny;
     C.P = k.ny + 2;  // padded column stride
+    C.last = k.nx * C.P + k.ny;
     C.inv_v = k.inv_v;
     C.cfl = (float)a.cfl;
     C.barrier = a.d_phi != nullptr;
@@ -488,14 +728,17 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
 
     LaneState s;
     s.pid = -1;
-    s.ix = s.iy = s.steps = s.stop_at = s.spc = 0;
-    s.o.x = s.o.y = s.v.x = s.v.y = s.qm = 0.f;
+    s.cx = s.cy = s.steps = s.stop_at = s.spc = 0;
+    s.u.x = s.u.y = s.v.x = s.v.y = s.hq = 0.f;
     s.clock = 0u;
     s.elapsed = 0.f;
     LaneTally t = {0u, 0u, 0u, 0u, 0u, 0u};
-    QuadCache q;
+    QuadCache q;          // always a quad of the grid: an inactive lane reads its fields too
     q.base = -1;
     q.c00 = q.c01 = q.c10 = q.c11 = tb_fcell{0.f, 0.f};
+    q.load(C.F, 0, C.P, C.last);
+    q.mark_open();
+    bool active = false;   // the lane holds a particle that is not waiting for a decision step
     bool open = true;
     // The warp's reserved block of claim ranks [wc, we): empty lanes are refilled from it
     // without an atomic, and a new block is reserved only when it runs short.  While the
@@ -508,11 +751,13 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
     const unsigned long long warps_all = (unsigned long long)gridDim.x * (blockDim.x >> 5);
 
     for (;;) {
-        unsigned need = __ballot_sync(FULL, s.pid < 0);
-        if (need != 0u) {
-            if (!open && wc >= we) {
-                if (pool != nullptr || need == FULL) break;
-            } else {
+        const bool closed = !open && wc >= we;
+        if (closed || __popc(__ballot_sync(FULL, !active)) >= WAIT_LANES) {
+            step_held<SMEM, RF>(k, C, s, t, q, active);
+            const unsigned need = __ballot_sync(FULL, s.pid < 0);
+            if (closed) {
+                if (need != 0u && (pool != nullptr || need == FULL)) break;
+            } else if (need != 0u) {
                 const unsigned cnt = __popc(need);
                 const unsigned long long avail = we - wc;
                 const bool reserve = avail < cnt && open;
@@ -556,12 +801,11 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
                         // converted by the scatter with the expressions below
                         const uint4 r0 = __ldg(k.rec + 2 * rank), r1 = __ldg(k.rec + 2 * rank + 1);
                         s.pid = (int)r0.x;
-                        q.base = -1;
-                        s.ix = (int)(r0.y & 0xffffu);
-                        s.iy = (int)r0.y >> 16;  // arithmetic shift keeps a negative row
-                        s.o = make_float2(__uint_as_float(r0.z), __uint_as_float(r0.w));
+                        s.cx = (int)(r0.y & 0xffffu);
+                        s.cy = (int)(r0.y >> 16);
+                        s.u = make_float2(__uint_as_float(r0.z), __uint_as_float(r0.w));
                         s.v = make_float2(__uint_as_float(r1.x), __uint_as_float(r1.y));
-                        s.qm = __uint_as_float(r1.z);
+                        s.hq = __uint_as_float(r1.z);
                         s.spc = (int)(r1.w >> 31);
                         s.steps = (int)(r1.w & 0x7fffffffu);
                         s.stop_at = min(a.max_steps, s.steps + a.step_budget);
@@ -572,17 +816,10 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
                     if (!REC && idx < n_all && a.d_status[idx] == 3 && a.d_steps[idx] < a.max_steps) {
                         const int pid = (int)idx;
                         s.pid = pid;
-                        q.base = -1;
-                        // metres -> cells: x lies in cell min(int(x/dx), nx-1) as in the
-                        // reference (trench_charging_2d.py:611)
-                        const double xc = a.d_x[pid] * k.inv_dx, yc = a.d_y[pid] * k.inv_dx;
-                        s.ix = min(max((int)xc, 0), C.nx - 1);
-                        s.iy = min((int)floor(yc), C.ny - 1);  // a start above the grid escapes at once
-                        s.o.x = fminf(fmaxf((float)(xc - (double)s.ix), 0.f), ONE_BELOW);
-                        s.o.y = fminf(fmaxf((float)(yc - (double)s.iy), 0.f), ONE_BELOW);
+                        start_position(a.d_x[pid], a.d_y[pid], k.inv_dx, C.nx, C.ny, &s.cx, &s.cy, &s.u);
                         s.v.x = (float)(a.d_vx[pid] * k.inv_v64);
                         s.v.y = (float)(a.d_vy[pid] * k.inv_v64);
-                        s.qm = (float)a.d_qm[pid];
+                        s.hq = (float)(0.5 * a.d_qm[pid]);
                         s.spc = a.d_spc[pid];
                         s.steps = a.d_steps[pid];
                         s.stop_at = min(a.max_steps, s.steps + a.step_budget);
@@ -594,21 +831,19 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
                             s.elapsed = (float)a.d_clock[2 * pid + 1];
                         }
                     }
+                    active = s.pid >= 0;
+                    if (active) {
+                        q.base = -1;
+                        q.load(C.F, s.cx * C.P + s.cy, C.P, C.last);
+                    }
                 }
                 wc = nwc;
                 we = nwe;
+                if (__ballot_sync(FULL, active) == 0u) continue;   // ranks of particles not to be traced
             }
-            need = __ballot_sync(FULL, s.pid < 0);
         }
-        if (need == 0u) {
-            // every lane holds a particle: step them all until one of them ends, one vote
-            // per step instead of the refill bookkeeping
-            do {
-                step_particle<SMEM, RF>(k, C, s, t, q);
-            } while (__all_sync(FULL, s.pid >= 0));
-        } else if (s.pid >= 0) {
-            step_particle<SMEM, RF>(k, C, s, t, q);
-        }
+        step_warp<SMEM, RF>(k, C, s, t, q, active, 0x7fffffff,
+                            closed ? __popc(__ballot_sync(FULL, active)) : 33 - WAIT_LANES);
     }
 
     if (pool != nullptr) {
@@ -624,14 +859,21 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
             __syncthreads();
             const int live = s_live;
             if (live == 0) break;
-            if ((int)threadIdx.x < live) pool_get<RF>(pool, T, threadIdx.x, s);
-            q.base = -1;
+            if ((int)threadIdx.x < live) {
+                pool_get<RF>(pool, T, threadIdx.x, s);
+                q.base = -1;
+                q.load(C.F, s.cx * C.P + s.cy, C.P, C.last);
+            } else {
+                q.mark_open();
+            }
+            active = s.pid >= 0;
             __syncthreads();
             if (threadIdx.x == 0) s_live = 0;
             if ((int)(threadIdx.x & ~31u) < live) {  // warp-uniform: this warp holds particles
-                for (int r = 0; r < TAIL_ROUND_STEPS; ++r) {
-                    if (__ballot_sync(FULL, s.pid >= 0) == 0u) break;
-                    if (s.pid >= 0) step_particle<SMEM, RF>(k, C, s, t, q);
+                int left = TAIL_ROUND_STEPS;
+                while (left > 0 && __any_sync(FULL, active)) {
+                    left -= step_warp<SMEM, RF>(k, C, s, t, q, active, left, __popc(__ballot_sync(FULL, active)));
+                    step_held<SMEM, RF>(k, C, s, t, q, active);
                 }
             }
         }
@@ -880,15 +1122,14 @@ K32 make_k32(const tb_ctx *ctx, const tb_trace_args *a) {
     k.rf_field = ctx->d_rf_field;
     k.rf_barrier = ctx->d_rf_barrier;
     k.rf_wave = ctx->d_rf_wave;
-    k.t_clock = k.wave_scale = k.t_sec = k.dt_max = k.bvs = k.bvm = 0.f;
-    k.n_phase_m1 = 0;
+    k.t_clock = k.t_sec = k.dt_max = k.bvs = k.bvm = 0.f;
+    k.short_steps = false;
     if (a->n_phase > 0) {
         // step time unit dx / vscale: in seconds, in clock units, and the in-flight step bound
         const double unit = ctx->dx / ctx->vscale;
         k.t_sec = (float)unit;
         k.t_clock = (float)(unit / a->period * 4294967296.0);
-        k.wave_scale = (float)(a->n_phase * 0x1p-32);
-        k.n_phase_m1 = a->n_phase - 1;
+        k.short_steps = a->dt_max < 0.5 * a->period;
         k.dt_max = (float)(a->dt_max / unit);
         k.bvs = (float)a->bound_vs;
         k.bvm = (float)a->bound_vm;
@@ -1058,16 +1299,14 @@ __device__ __forceinline__ void claim_scatter_body(const K32 &k, int b, int nb) 
             const int32_t n_steps = a.d_steps[i];
             const int8_t sp = a.d_spc[i];
             c = claim_class(kk, ion_class);
-            const double xc = x * k.inv_dx, yc = y * k.inv_dx;
-            const int ix = min(max((int)xc, 0), k.nx - 1);
-            const int iy = min((int)floor(yc), k.ny - 1);
-            const float ox = fminf(fmaxf((float)(xc - (double)ix), 0.f), ONE_BELOW);
-            const float oy = fminf(fmaxf((float)(yc - (double)iy), 0.f), ONE_BELOW);
+            int cx, cy;
+            float2 u;
+            start_position(x, y, k.inv_dx, k.nx, k.ny, &cx, &cy, &u);
             const float vx = (float)(vx64 * k.inv_v64), vy = (float)(vy64 * k.inv_v64);
-            const float qm = (float)qm64;
-            r0 = make_uint4((unsigned)i, ((unsigned)ix & 0xffffu) | ((unsigned)iy << 16), __float_as_uint(ox),
-                            __float_as_uint(oy));
-            r1 = make_uint4(__float_as_uint(vx), __float_as_uint(vy), __float_as_uint(qm),
+            const float hq = (float)(0.5 * qm64);
+            r0 = make_uint4((unsigned)i, (unsigned)cx | ((unsigned)cy << 16), __float_as_uint(u.x),
+                            __float_as_uint(u.y));
+            r1 = make_uint4(__float_as_uint(vx), __float_as_uint(vy), __float_as_uint(hq),
                             (unsigned)n_steps | (sp ? 0x80000000u : 0u));
         }
         const unsigned peers = __match_any_sync(0xffffffffu, c);
