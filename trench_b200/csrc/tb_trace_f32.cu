@@ -7,15 +7,16 @@
 //  * Position = nearest grid vertex (integers) + FP32 offset in [-0.5, 0.5] cells, so the
 //    index and the periodic wrap are exact integer operations, the offset keeps 2^-25-cell
 //    resolution everywhere in the grid, and the vertex is the index of the bilinear quad.
+//    With the field in global memory: cell + offset in [0, 1) (see LaneState).
 //  * Velocities in units of vscale (m/s); time in dx/vscale; the packed field is
 //    E*vac*dx/vscale^2 so qm*field is the acceleration in these units.
 //  * The packed field (8 bytes per cell, vacuum flag in bit 0 of Ex) is staged
 //    once per block into shared memory with a bulk async copy (TMA engine,
 //    cp.async.bulk + mbarrier); every bilinear gather is a shared-memory load.  A lane
 //    keeps its quad's corners in registers and loads only when it changes quad.
-//    Grids too large for shared memory read the same layout from global memory
-//    (L2-resident).
-//  * Three forms of a step.  While every active lane of a warp is in an open quad (no
+//    Grids too large for shared memory, and small batches, read the same layout from
+//    global memory (L2-resident).
+//  * Three forms of a step (field in shared memory).  While every active lane of a warp is in an open quad (no
 //    solid corner, not at the top or bottom edge) the warp runs step_open, which has no
 //    branch; with any lane near a wall it runs step_near, whose extra arithmetic is
 //    branch-free too; a step that meets a wall, a corner or the edge is not taken there but
@@ -63,6 +64,7 @@ struct K32 {
     int bytes;                      // packed field bytes (multiple of 16)
     int pool_off;                   // byte offset of the drain pool in dynamic shared memory, -1 = none
     int reverse;                    // claim particles from the last index down
+    bool cell_frame;                // claim records hold cell and offset (see LaneState)
     // learned claim order (nullptr rec = none): claim records in claim order, their number,
     // each particle's key, the ion bins' classes, per-block class starts, per-bin step sums,
     // 1 / domain width and the ordering kernels' blocks
@@ -83,6 +85,7 @@ struct K32 {
     const float4 *rf_wave;          // (vs_i, vm_i, vs_i+1 - vs_i, vm_i+1 - vm_i), i < n_phase
     float t_clock;                  // clock units (2^-32 period) per unit of step time
     bool short_steps;               // every step is under half a period (clock steps fit 32 bits)
+    float wave_scale;               // n_phase * 2^-32: clock -> table position (cell frame)
     float t_sec;                    // seconds per unit of step time (dx / vscale)
     float dt_max;                   // step bound of the in-flight field, in step time
     float bvs, bvm;                 // largest voltage deltas of the waveform
@@ -154,6 +157,12 @@ __device__ bool stage_field(void *dst, const void *src, int bytes, uint64_t *mba
 // cx in [0, nx] (0 and nx are the same vertex), cy in [0, ny]; a particle below the grid (open
 // bottom rows only) has cy = 0 and the rest of its distance in u.y.  Velocity in vscale units;
 // hq is half the charge-to-mass ratio.  pid < 0 = no particle.
+// Fields in global memory (SMEM = false): the cell frame -- cx, cy is the particle's cell (cy < 0
+// below the grid), u in [0, 1) its offset in it, hq the whole charge-to-mass ratio.  The vertex
+// frame and its three forms of a step measured 2650 against 3150 us a batch there (200 x 700
+// cells, 2^19 particles), with as many particles that end elsewhere than in FP64 (163 and 158 of
+// 3.1e6), but not the same ones: on so fine a grid each one moves the batch's potential by
+// more than batches may differ.
 struct LaneState {
     int pid, cx, cy, steps, stop_at, spc;
     float2 u, v;                    // offset and velocity, packed pairs
@@ -177,18 +186,32 @@ __device__ __forceinline__ void vertex_of(double xc, int cell, int *c, float *u)
     *c = cell + h;
     *u = (float)(d - (double)h);
 }
-__device__ __forceinline__ void start_position(const double x, const double y, double inv_dx, int nx, int ny, int *cx,
-                                               int *cy, float2 *u) {
+constexpr float ONE_BELOW = 0x1.fffffep-1f;  // largest float < 1
+__device__ __forceinline__ void start_position(const double x, const double y, double inv_dx, int nx, int ny,
+                                               bool cell_frame, int *cx, int *cy, float2 *u) {
     // x lies in cell min(int(x/dx), nx-1) as in the reference (trench_charging_2d.py:611); a
     // start above the grid escapes at once
     const double xc = x * inv_dx, yc = y * inv_dx;
-    vertex_of(xc, min(max((int)xc, 0), nx - 1), cx, &u->x);
+    const int ix = min(max((int)xc, 0), nx - 1);
+    if (cell_frame) {
+        const int iy = min((int)floor(yc), ny - 1);
+        *cx = ix;
+        *cy = iy;
+        u->x = fminf(fmaxf((float)(xc - (double)ix), 0.f), ONE_BELOW);
+        u->y = fminf(fmaxf((float)(yc - (double)iy), 0.f), ONE_BELOW);
+        return;
+    }
+    vertex_of(xc, ix, cx, &u->x);
     if (yc < 0.0) {
         *cy = 0;
         u->y = (float)fmax(yc, -1e6);
     } else {
         vertex_of(yc, min((int)yc, ny - 1), cy, &u->y);
     }
+}
+// Half the charge-to-mass ratio (vertex frame) or all of it (cell frame).
+__device__ __forceinline__ float charge_of(double qm, bool cell_frame) {
+    return cell_frame ? (float)qm : (float)(0.5 * qm);
 }
 
 // The four bilinear corners of a lane's quad and their base index (-1 = none).  A step
@@ -205,7 +228,7 @@ struct QuadCache {
     // or velocity that is not finite may hold any index)
     template <bool SMEM>
     __device__ __forceinline__ void load(const FieldView<SMEM> &F, int at, int P, int last) {
-        const int b = (int)min((unsigned)at, (unsigned)last);
+        const int b = SMEM ? (int)min((unsigned)at, (unsigned)last) : at;
         if (SMEM) {
             // predicated in place: a branch around the loads costs more than the loads
             const uint32_t a0 = F.shared_address() + 8u * (unsigned)b, a1 = a0 + 8u * (unsigned)P;
@@ -234,7 +257,8 @@ struct LaneTally {
     unsigned steps, esc_i, esc_e, lost, hit_i, hit_e;
 };
 
-// The quad flag of a quad's lower-left corner: all four cells vacuum, and no step leaves the grid.
+// The quad flag of a quad's lower-left corner (tb_quad_vacuum): all four cells vacuum and, in
+// shared memory, no step leaves the grid.
 __device__ __forceinline__ bool is_open(const tb_fcell &c00) { return __float_as_uint(c00.ey) & 1u; }
 
 // Loop-invariant parameters of one case.
@@ -306,12 +330,228 @@ __device__ __forceinline__ void finish_particle(const K32 &k, LaneState &s, Lane
     s.pid = -1;
 }
 
+// Quad of a particle: its vertex, or in the cell frame the vertex nearest to its offset.
+template <bool SMEM>
+__device__ __forceinline__ void load_quad(const CaseView<SMEM> &C, const LaneState &s, QuadCache &q) {
+    int at = s.cx * C.P + s.cy;
+    if (!SMEM) at = (s.cx + (s.u.x >= 0.5f ? 1 : 0)) * C.P + max(s.cy + (s.u.y >= 0.5f ? 1 : 0), 0);
+    q.load(C.F, at, C.P, C.last);
+}
+
+// ---- the cell frame: fields in global memory ---------------------------------------------
+
+// Waveform table position of a clock: interval i and the position within it.
+__device__ __forceinline__ int cell_rf_interval(const K32 &k, uint32_t clock, float &w) {
+    const float f = (float)clock * k.wave_scale;
+    const int i = min((int)f, k.a.n_phase - 1);  // a clock just below 2^32 may round up to n
+    w = f - (float)i;
+    return i;
+}
+
+// Acceleration A, time step and clock advance of the next step (see step_size).
+template <bool RF>
+__device__ __forceinline__ void cell_step_size(const K32 &k, const CaseView<false> &C, const LaneState &s,
+                                               const QuadCache &q, bool near, float2 &A, float &dt, uint32_t &inc) {
+    const float2 tq = __fadd2_rn(s.u, make_float2(s.u.x >= 0.5f ? -0.5f : 0.5f, s.u.y >= 0.5f ? -0.5f : 0.5f));
+    const float tx = tq.x, ty = tq.y;
+    const tb_fcell c00 = q.c00, c01 = q.c01, c10 = q.c10, c11 = q.c11;
+    const float2 E = bilinear2(make_float2(c00.ex, c00.ey), make_float2(c01.ex, c01.ey), make_float2(c10.ex, c10.ey),
+                               make_float2(c11.ex, c11.ey), make_float2(tx, tx), make_float2(ty, ty));
+    float inv_sw = 1.f;
+    if (near) {
+        const float v00 = vac_of(c00), v01 = vac_of(c01), v10 = vac_of(c10), v11 = vac_of(c11);
+        const float s0 = fmaf(ty, v01 - v00, v00), s1 = fmaf(ty, v11 - v10, v10);
+        inv_sw = __fdividef(1.f, fmaxf(fmaf(tx, s1 - s0, s0), 1e-12f));
+    }
+    const float speed = sqrtf(fmaf(s.v.x, s.v.x, s.v.y * s.v.y));
+    const float qs = s.hq * inv_sw;
+    inc = 0u;
+    if (!RF) {
+        A = __fmul2_rn(make_float2(qs, qs), E);
+        const float acc = sqrtf(fmaf(A.x, A.x, A.y * A.y));
+        dt = __fdividef(C.cfl, speed + sqrtf(2.f * acc) + C.inv_v);
+    } else {
+        // in-flight RF field (trench_trace.cu:97-110), as step_size
+        const int base = q.base, P = C.P;
+        const float ux = 1.f - tx, uy = 1.f - ty;
+        const float w00 = ux * uy, w10 = tx * uy, w01 = ux * ty, w11 = tx * ty;
+        const uint32_t c0 = s.clock;
+        float w0;
+        const int i0 = cell_rf_interval(k, c0, w0);
+        const float4 e0 = __ldg(k.rf_wave + i0);
+        const float4 b00 = __ldg(k.rf_field + base), b01 = __ldg(k.rf_field + base + 1);
+        const float4 b10 = __ldg(k.rf_field + base + P), b11 = __ldg(k.rf_field + base + P + 1);
+        const float sxs = w00 * b00.x + w10 * b10.x + w01 * b01.x + w11 * b11.x;
+        const float sys = w00 * b00.y + w10 * b10.y + w01 * b01.y + w11 * b11.y;
+        const float sxm = w00 * b00.z + w10 * b10.z + w01 * b01.z + w11 * b11.z;
+        const float sym = w00 * b00.w + w10 * b10.w + w01 * b01.w + w11 * b11.w;
+        const float bx = fabsf(E.x) + (k.bvs * fabsf(sxs) + k.bvm * fabsf(sxm));
+        const float by = fabsf(E.y) + (k.bvs * fabsf(sys) + k.bvm * fabsf(sym));
+        const float accel = fabsf(s.hq) * inv_sw * sqrtf(bx * bx + by * by);
+        dt = fminf(k.dt_max, __fdividef(C.cfl, speed + sqrtf(2.f * accel) + C.inv_v));
+        uint32_t mid;
+        if (k.short_steps) {
+            inc = __float2uint_rn(dt * k.t_clock);
+            mid = c0 + (inc >> 1);
+        } else {
+            const unsigned long long w64 = __float2ull_rn(dt * k.t_clock);
+            inc = (uint32_t)w64;
+            mid = c0 + (uint32_t)(w64 >> 1);
+        }
+        float w;
+        const int im = cell_rf_interval(k, mid, w);
+        const float4 e = im == i0 ? e0 : __ldg(k.rf_wave + im);
+        const float vs = fmaf(w, e.z, e.x), vm = fmaf(w, e.w, e.y);
+        A = make_float2(qs * (E.x + (vs * sxs + vm * sxm)), qs * (E.y + (vs * sys + vm * sym)));
+    }
+}
+
+// v' = v + a dt and the move (v + v') dt / 2 = (v + a dt / 2) dt.  A step moves less than one cell, so
+// the new offset lies in (-1, 2): the cell change is its floor and the new offset the
+// remainder (a remainder that rounds up to 1 is clamped below 1).  Compares in place of the
+// floors and conversions: 3150 -> 3280 us a batch (200 x 700 cells, 2^19 particles).
+struct CellMove {
+    float2 v, S, o;
+    int dix, nix, niy;
+};
+// a + b, never contracted with the product that made b (an add with a rounding modifier is not).
+__device__ __forceinline__ float2 add2_alone(float2 a, float2 b) {
+    float2 r;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+        "add.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ CellMove cell_move(const CaseView<false> &C, const LaneState &s, float2 A, float dt) {
+    CellMove m;
+    const float2 dtt = make_float2(dt, dt);
+    const float hdt = 0.5f * dt;
+    m.v = __ffma2_rn(A, dtt, s.v);
+    m.S = __fmul2_rn(__ffma2_rn(A, make_float2(hdt, hdt), s.v), dtt);
+    const float2 pos = add2_alone(s.u, m.S);
+    const float fnx = floorf(pos.x), fny = floorf(pos.y);
+    const float2 rem = __ffma2_rn(make_float2(fnx, fny), make_float2(-1.f, -1.f), pos);
+    m.o = make_float2(fminf(rem.x, ONE_BELOW), fminf(rem.y, ONE_BELOW));
+    m.dix = (int)fnx;
+    const int nix = s.cx + m.dix;
+    m.nix = nix < 0 ? C.nx - 1 : (nix >= C.nx ? 0 : nix);
+    m.niy = s.cy + (int)fny;
+    return m;
+}
+
+// One step of one particle (trench_charging_2d.py:584-650), as step_open and step_decide
+// together; these steps wait for the field's loads, and one branch a step costs less than the
+// lanes that three forms hold back.
+template <bool RF>
+__device__ __forceinline__ void cell_step(const K32 &k, const CaseView<false> &C, LaneState &s, LaneTally &t,
+                                          QuadCache &q) {
+    const tb_trace_args &a = k.a;
+    const int ny = C.ny, P = C.P;
+    load_quad(C, s, q);
+    // a step below half a cell ends in a corner cell of its quad
+    const bool near = !(C.small_steps && is_open(q.c00));
+    float2 A;
+    float dt;
+    uint32_t inc;
+    cell_step_size<RF>(k, C, s, q, near, A, dt, inc);
+    const CellMove m = cell_move(C, s, A, dt);
+    if (RF) {
+        s.clock += inc;
+        s.elapsed += dt * k.t_sec;
+    }
+    ++s.steps;
+    const bool escaped = m.niy >= ny;
+    bool hit = false, corner = false;
+    if (near && !escaped) {
+        hit = !C.F.vac((m.nix + 1) * P + max(m.niy, -1) + 1);
+        // both the column and the (clipped) row changed: a staircase corner may lie on the path
+        // between two vacuum cells (trench_charging_2d.py:614-621).  The move reaches the wall
+        // only if the cell beyond the first boundary crossed is solid (the first-face rule
+        // below, same expressions).
+        corner = C.tapered && !hit && m.dix != 0 && max(m.niy, 0) != max(s.cy, 0);
+        if (corner) {
+            const int y0c = min(max(s.cy, 0), ny - 1), iyn = min(max(m.niy, 0), ny - 1);
+            const float fx = ((m.dix > 0 ? 1.f : 0.f) - s.u.x) / m.S.x;
+            const float fy = ((iyn > y0c ? 1.f : 0.f) - s.u.y) / m.S.y;
+            const bool x_first = fx < fy;
+            corner = !C.F.vac((x_first ? m.nix + 1 : s.cx + 1) * P + (x_first ? y0c : iyn) + 1);
+        }
+    }
+    if (!(hit || corner || escaped || s.steps >= s.stop_at)) {
+        s.cx = m.nix; s.cy = m.niy; s.u = m.o; s.v = m.v;
+        return;
+    }
+
+    // wall contact, escape or step cap
+    const int y0c = min(max(s.cy, 0), ny - 1), iyn = min(max(m.niy, 0), ny - 1);
+    const int diy = iyn - y0c;       // rows clipped like the reference
+    int dcell = m.nix * ny + iyn;
+    bool reflected = false;
+    if (hit ? C.first_face : corner) {
+        // first solid face crossed (trench_charging_2d.py:512-539) in cell units
+        const float inf = __int_as_float(0x7f800000);
+        const float fx = m.dix != 0 ? ((m.dix > 0 ? 1.f : 0.f) - s.u.x) / m.S.x : inf;
+        const float fy = diy != 0 ? ((diy > 0 ? 1.f : 0.f) - s.u.y) / m.S.y : inf;
+        const bool x_first = fx < fy;
+        const int ax_ = x_first ? m.nix : s.cx, ay_ = x_first ? y0c : y0c + diy;
+        const bool use_last = m.dix != 0 && diy != 0 && C.F.vac((ax_ + 1) * P + ay_ + 1);
+        const int cx = use_last ? m.nix : ax_, cy = use_last ? y0c + diy : ay_;
+        const bool face_x = use_last ? !x_first : x_first;
+        const int ccell = cx * ny + cy;
+        hit = !C.F.vac((cx + 1) * P + cy + 1);
+        dcell = ccell;
+        if (hit && C.barrier) {
+            const float4 b = __ldg(k.barrier + ccell);
+            // neighbour the particle came from: W/E across an x face, S/N across a y face
+            float dphi = face_x ? (m.dix > 0 ? b.x : b.y) : (diy > 0 ? b.z : b.w);
+            if (RF) {
+                // barrier of the instantaneous potential at the clock after the step
+                // (trench_trace.cu:131-136)
+                float w;
+                const float4 e = __ldg(k.rf_wave + cell_rf_interval(k, s.clock, w));
+                const float vs = fmaf(w, e.z, e.x), vm = fmaf(w, e.w, e.y);
+                const float4 bs = __ldg(k.rf_barrier + ccell), bm = __ldg(k.rf_barrier + C.cells + ccell);
+                const float ds = face_x ? (m.dix > 0 ? bs.x : bs.y) : (diy > 0 ? bs.z : bs.w);
+                const float dm = face_x ? (m.dix > 0 ? bm.x : bm.y) : (diy > 0 ? bm.z : bm.w);
+                dphi += vs * ds + vm * dm;
+            }
+            const float vn = face_x ? m.v.x : m.v.y;
+            if (0.5f * vn * vn < s.hq * dphi) {
+                // reflect: the normal velocity flips, the position stays at the start point
+                s.v.x = face_x ? -m.v.x : m.v.x;
+                s.v.y = face_x ? m.v.y : -m.v.y;
+                hit = false;
+                reflected = true;
+            }
+        }
+    }
+    if (!reflected) { s.cx = m.nix; s.cy = m.niy; s.u = m.o; s.v = m.v; }
+    if (hit) {
+        if (dcell < 0 || dcell >= C.cells) {
+            atomicCAS(k.err, TB_DERR_NONE, TB_DERR_BAD_CELL);
+        } else {
+            tb_deposit(a.d_counts, (size_t)s.spc * C.cells + dcell);
+        }
+        if (a.d_hit) a.d_hit[s.pid] = dcell;
+        if (s.spc == 0) ++t.hit_i; else ++t.hit_e;
+        finish_particle<RF>(k, s, t, 1);
+    } else if (escaped && !reflected) {
+        if (s.spc == 0) ++t.esc_i; else ++t.esc_e;
+        finish_particle<RF>(k, s, t, 2);
+    } else if (s.steps >= s.stop_at) {
+        finish_particle<RF>(k, s, t, 3);
+    }
+}
+
+// ---- the vertex frame: fields in shared memory -------------------------------------------
+
 // Half acceleration h, time step and (circuit_rf) clock advance of a particle's next step
 // (trench_charging_2d.py:492-509, 587-608): vacuum-weighted bilinear field and the CFL step
 // dt = cfl / (|v| + sqrt(2 |a|) + 1 m/s), with sqrt(2 |a|) = 2 (|h|^2)^(1/4).  NEAR: the quad may
 // hold solid corners, whose weights are left out; otherwise the vacuum weights sum to one.
-template <bool SMEM, bool RF, bool NEAR>
-__device__ __forceinline__ void step_size(const K32 &k, const CaseView<SMEM> &C, const LaneState &s,
+template <bool RF, bool NEAR>
+__device__ __forceinline__ void step_size(const K32 &k, const CaseView<true> &C, const LaneState &s,
                                           const QuadCache &q, float2 &h, float &dt, uint32_t &inc) {
     const float tx = s.u.x + 0.5f, ty = s.u.y + 0.5f;
     const float2 txx = make_float2(tx, tx), tyy = make_float2(ty, ty);
@@ -389,8 +629,8 @@ __device__ __forceinline__ int wrap_vertex(int c, int nx) {
 }
 
 // Takes a step of length dt to offset p (r = rounded(p)) from the present vertex.
-template <bool SMEM, bool RF>
-__device__ __forceinline__ void take_step(const K32 &k, const CaseView<SMEM> &C, LaneState &s, QuadCache &q, float2 h,
+template <bool RF>
+__device__ __forceinline__ void take_step(const K32 &k, const CaseView<true> &C, LaneState &s, QuadCache &q, float2 h,
                                           float dt, uint32_t inc, float2 p, float2 r) {
     const float d2 = dt + dt;
     s.cx = wrap_vertex(s.cx + vertex_change(r.x), C.nx);
@@ -401,38 +641,38 @@ __device__ __forceinline__ void take_step(const K32 &k, const CaseView<SMEM> &C,
         s.clock += inc;
         s.elapsed += dt * k.t_sec;
     }
-    q.load(C.F, s.cx * C.P + s.cy, C.P, C.last);
+    load_quad(C, s, q);
 }
 
 // A step of a warp whose lanes' quads are all open: a step moves at most cfl cells (|v| dt +
 // |a| dt^2 / 2 <= cfl for the CFL dt), so with cfl below one half it ends in one of the quad's
 // four corner cells, all vacuum.  Inactive lanes take a step of length zero, which leaves them
 // exactly as they are.
-template <bool SMEM, bool RF>
-__device__ __forceinline__ void step_open(const K32 &k, const CaseView<SMEM> &C, LaneState &s, QuadCache &q,
+template <bool RF>
+__device__ __forceinline__ void step_open(const K32 &k, const CaseView<true> &C, LaneState &s, QuadCache &q,
                                           bool active) {
     float2 h;
     float dt;
     uint32_t inc;
-    step_size<SMEM, RF, false>(k, C, s, q, h, dt, inc);
+    step_size<RF, false>(k, C, s, q, h, dt, inc);
     if (!active) {
         dt = 0.f;
         inc = 0u;
     }
     const float2 p = moved(s, h, dt);
-    take_step<SMEM, RF>(k, C, s, q, h, dt, inc, p, rounded(p));
+    take_step<RF>(k, C, s, q, h, dt, inc, p, rounded(p));
 }
 
 // A step of a warp with lanes near a wall or an edge of the grid.  It is taken if it ends in a
 // vacuum cell of the grid with no staircase corner on the way; otherwise the particle stays as
 // it was and the return is false: the step needs the decisions of step_decide.
-template <bool SMEM, bool RF>
-__device__ __forceinline__ bool step_near(const K32 &k, const CaseView<SMEM> &C, LaneState &s, QuadCache &q,
+template <bool RF>
+__device__ __forceinline__ bool step_near(const K32 &k, const CaseView<true> &C, LaneState &s, QuadCache &q,
                                           bool active) {
     float2 h;
     float dt;
     uint32_t inc;
-    step_size<SMEM, RF, true>(k, C, s, q, h, dt, inc);
+    step_size<RF, true>(k, C, s, q, h, dt, inc);
     float2 p = moved(s, h, dt), r = rounded(p);
     bool go;
     if (C.small_steps) {
@@ -458,21 +698,21 @@ __device__ __forceinline__ bool step_near(const K32 &k, const CaseView<SMEM> &C,
         p = s.u;
         r = make_float2(MAGIC, MAGIC);
     }
-    take_step<SMEM, RF>(k, C, s, q, h, dt, inc, p, r);
+    take_step<RF>(k, C, s, q, h, dt, inc, p, r);
     return go;
 }
 
 // One step of one particle with everything it may meet (trench_charging_2d.py:584-650):
 // escape, staircase corner, first-face wall entry, barrier reflection, the step cap (s.steps
 // counts the step already); an ended particle's outputs are written and s.pid becomes -1.
-template <bool SMEM, bool RF>
-__device__ __forceinline__ void step_decide(const K32 &k, const CaseView<SMEM> &C, LaneState &s, LaneTally &t,
+template <bool RF>
+__device__ __forceinline__ void step_decide(const K32 &k, const CaseView<true> &C, LaneState &s, LaneTally &t,
                                             QuadCache &q) {
     const int nx = C.nx, ny = C.ny, P = C.P;
     float2 h;
     float dt;
     uint32_t inc;
-    step_size<SMEM, RF, true>(k, C, s, q, h, dt, inc);
+    step_size<RF, true>(k, C, s, q, h, dt, inc);
     const bool near = !(C.small_steps && is_open(q.c00));
     const float2 p = moved(s, h, dt), r = rounded(p);
     const float dd = dt * dt, d2 = dt + dt;
@@ -563,7 +803,7 @@ __device__ __forceinline__ void step_decide(const K32 &k, const CaseView<SMEM> &
             s.clock += inc;
             s.elapsed += dt * k.t_sec;
         }
-        q.load(C.F, cxw * P + cyn, P, C.last);
+        load_quad(C, s, q);
     }
 
     if (hit) {
@@ -594,7 +834,7 @@ constexpr int TAIL_ROUND_STEPS = 64;
 template <bool RF>
 __device__ __forceinline__ void pool_put(uint32_t *P, int T, int q, const LaneState &s) {
     P[0 * T + q] = (uint32_t)s.pid;
-    P[1 * T + q] = (uint32_t)s.cx | ((uint32_t)s.cy << 16);
+    P[1 * T + q] = ((uint32_t)s.cx & 0xffffu) | ((uint32_t)s.cy << 16);
     P[2 * T + q] = (uint32_t)s.steps;
     P[3 * T + q] = (uint32_t)s.stop_at | ((uint32_t)s.spc << 31);
     P[4 * T + q] = __float_as_uint(s.u.x);
@@ -613,7 +853,7 @@ __device__ __forceinline__ void pool_get(const uint32_t *P, int T, int q, LaneSt
     s.pid = (int)P[0 * T + q];
     const uint32_t xy = P[1 * T + q];
     s.cx = (int)(xy & 0xffffu);
-    s.cy = (int)(xy >> 16);
+    s.cy = (int)xy >> 16;   // arithmetic shift keeps a negative row
     s.steps = (int)P[2 * T + q];
     const uint32_t w = P[3 * T + q];
     s.stop_at = (int)(w & 0x7fffffffu);
@@ -634,8 +874,8 @@ __device__ __forceinline__ void pool_get(const uint32_t *P, int T, int q, LaneSt
 // after `limit` steps; particles at their cap end here.  Returns the steps made.  Every lane
 // of the warp calls it.  While every active lane's quad is open the whole warp runs step_open,
 // which has no branch; the cached quad of an inactive lane is marked open.
-template <bool SMEM, bool RF>
-__device__ __forceinline__ int step_warp(const K32 &k, const CaseView<SMEM> &C, LaneState &s, LaneTally &t,
+template <bool RF>
+__device__ __forceinline__ int step_warp(const K32 &k, const CaseView<true> &C, LaneState &s, LaneTally &t,
                                          QuadCache &q, bool &active, int limit, int least) {
     const unsigned FULL = 0xffffffffu;
     const int n = (int)min((unsigned)limit, __reduce_min_sync(FULL, active ? (unsigned)(s.stop_at - s.steps)
@@ -643,10 +883,10 @@ __device__ __forceinline__ int step_warp(const K32 &k, const CaseView<SMEM> &C, 
     int j = 0;
     for (;;) {
         if (C.small_steps && __all_sync(FULL, is_open(q.c00))) {
-            step_open<SMEM, RF>(k, C, s, q, active);
+            step_open<RF>(k, C, s, q, active);
             if (++j >= n) break;
         } else {
-            if (!step_near<SMEM, RF>(k, C, s, q, active) && active) {
+            if (!step_near<RF>(k, C, s, q, active) && active) {
                 s.steps += j;
                 active = false;
                 q.mark_open();
@@ -666,8 +906,8 @@ __device__ __forceinline__ int step_warp(const K32 &k, const CaseView<SMEM> &C, 
 }
 
 // The decision steps of the held lanes (occupied, not active).
-template <bool SMEM, bool RF>
-__device__ __forceinline__ void step_held(const K32 &k, const CaseView<SMEM> &C, LaneState &s, LaneTally &t,
+template <bool RF>
+__device__ __forceinline__ void step_held(const K32 &k, const CaseView<true> &C, LaneState &s, LaneTally &t,
                                           QuadCache &q, bool &active) {
     if (s.pid >= 0 && !active) {
         s.cx = min(max(s.cx, 0), C.nx);   // any index after steps that were not finite
@@ -677,9 +917,9 @@ __device__ __forceinline__ void step_held(const K32 &k, const CaseView<SMEM> &C,
             s.cy = 0;
         }
         q.base = -1;
-        q.load(C.F, s.cx * C.P + s.cy, C.P, C.last);
+        load_quad(C, s, q);
         ++s.steps;
-        step_decide<SMEM, RF>(k, C, s, t, q);
+        step_decide<RF>(k, C, s, t, q);
         active = s.pid >= 0;
         if (!active) q.mark_open();
     }
@@ -752,8 +992,8 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
 
     for (;;) {
         const bool closed = !open && wc >= we;
-        if (closed || __popc(__ballot_sync(FULL, !active)) >= WAIT_LANES) {
-            step_held<SMEM, RF>(k, C, s, t, q, active);
+        if (closed || __popc(__ballot_sync(FULL, !active)) >= (SMEM ? WAIT_LANES : 1)) {
+            if constexpr (SMEM) step_held<RF>(k, C, s, t, q, active);
             const unsigned need = __ballot_sync(FULL, s.pid < 0);
             if (closed) {
                 if (need != 0u && (pool != nullptr || need == FULL)) break;
@@ -802,7 +1042,7 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
                         const uint4 r0 = __ldg(k.rec + 2 * rank), r1 = __ldg(k.rec + 2 * rank + 1);
                         s.pid = (int)r0.x;
                         s.cx = (int)(r0.y & 0xffffu);
-                        s.cy = (int)(r0.y >> 16);
+                        s.cy = (int)r0.y >> 16;   // arithmetic: a row below the grid is negative
                         s.u = make_float2(__uint_as_float(r0.z), __uint_as_float(r0.w));
                         s.v = make_float2(__uint_as_float(r1.x), __uint_as_float(r1.y));
                         s.hq = __uint_as_float(r1.z);
@@ -816,10 +1056,10 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
                     if (!REC && idx < n_all && a.d_status[idx] == 3 && a.d_steps[idx] < a.max_steps) {
                         const int pid = (int)idx;
                         s.pid = pid;
-                        start_position(a.d_x[pid], a.d_y[pid], k.inv_dx, C.nx, C.ny, &s.cx, &s.cy, &s.u);
+                        start_position(a.d_x[pid], a.d_y[pid], k.inv_dx, C.nx, C.ny, !SMEM, &s.cx, &s.cy, &s.u);
                         s.v.x = (float)(a.d_vx[pid] * k.inv_v64);
                         s.v.y = (float)(a.d_vy[pid] * k.inv_v64);
-                        s.hq = (float)(0.5 * a.d_qm[pid]);
+                        s.hq = charge_of(a.d_qm[pid], !SMEM);
                         s.spc = a.d_spc[pid];
                         s.steps = a.d_steps[pid];
                         s.stop_at = min(a.max_steps, s.steps + a.step_budget);
@@ -832,18 +1072,27 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
                         }
                     }
                     active = s.pid >= 0;
-                    if (active) {
-                        q.base = -1;
-                        q.load(C.F, s.cx * C.P + s.cy, C.P, C.last);
-                    }
+                    q.base = -1;
+                    if (SMEM && active) load_quad(C, s, q);
                 }
                 wc = nwc;
                 we = nwe;
                 if (__ballot_sync(FULL, active) == 0u) continue;   // ranks of particles not to be traced
             }
         }
-        step_warp<SMEM, RF>(k, C, s, t, q, active, 0x7fffffff,
-                            closed ? __popc(__ballot_sync(FULL, active)) : 33 - WAIT_LANES);
+        if constexpr (SMEM) {
+            step_warp<RF>(k, C, s, t, q, active, 0x7fffffff,
+                          closed ? __popc(__ballot_sync(FULL, active)) : 33 - WAIT_LANES);
+        } else if (__all_sync(FULL, active)) {
+            // step all lanes until a particle ends, one vote per step
+            do {
+                cell_step<RF>(k, C, s, t, q);
+            } while (__all_sync(FULL, s.pid >= 0));
+            active = s.pid >= 0;
+        } else if (active) {
+            cell_step<RF>(k, C, s, t, q);
+            active = s.pid >= 0;
+        }
     }
 
     if (pool != nullptr) {
@@ -862,8 +1111,8 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
             if ((int)threadIdx.x < live) {
                 pool_get<RF>(pool, T, threadIdx.x, s);
                 q.base = -1;
-                q.load(C.F, s.cx * C.P + s.cy, C.P, C.last);
-            } else {
+                if (SMEM) load_quad(C, s, q);
+            } else if (SMEM) {
                 q.mark_open();
             }
             active = s.pid >= 0;
@@ -872,8 +1121,14 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
             if ((int)(threadIdx.x & ~31u) < live) {  // warp-uniform: this warp holds particles
                 int left = TAIL_ROUND_STEPS;
                 while (left > 0 && __any_sync(FULL, active)) {
-                    left -= step_warp<SMEM, RF>(k, C, s, t, q, active, left, __popc(__ballot_sync(FULL, active)));
-                    step_held<SMEM, RF>(k, C, s, t, q, active);
+                    if constexpr (SMEM) {
+                        left -= step_warp<RF>(k, C, s, t, q, active, left, __popc(__ballot_sync(FULL, active)));
+                        step_held<RF>(k, C, s, t, q, active);
+                    } else {
+                        if (active) cell_step<RF>(k, C, s, t, q);
+                        active = s.pid >= 0;
+                        --left;
+                    }
                 }
             }
         }
@@ -969,7 +1224,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
 }
 
 // Packs FP64 fields into the halo-padded FP32 tracer layout; one thread per cell.
-__global__ void pack_fields_kernel(int nx, int ny, double scale_e, double scale_phi, const uint8_t *vac,
+__global__ void pack_fields_kernel(int nx, int ny, bool edges, double scale_e, double scale_phi, const uint8_t *vac,
                                    const double *ex, const double *ey, const double *phi,
                                    const double *wface, tb_fcell *out, float4 *bar) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -977,7 +1232,7 @@ __global__ void pack_fields_kernel(int nx, int ny, double scale_e, double scale_
     if (c >= cells) return;
     const int ix = c / ny, iy = c - ix * ny;
     const int v = vac[c] ? 1 : 0;
-    tb_store_packed(out, vac, nx, ny, ix, iy, tb_pack_cell(ex[c], ey[c], v, scale_e));
+    tb_store_packed(out, vac, nx, ny, ix, iy, edges, tb_pack_cell(ex[c], ey[c], v, scale_e));
     float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
     if (!v && phi != nullptr) {
         const int w = (ix == 0 ? nx - 1 : ix - 1) * ny + iy;
@@ -1058,7 +1313,7 @@ int tb_launch_pack_fields(tb_ctx *ctx, const double *ex, const double *ey, const
     const double scale_phi = 1.0 / (vscale * vscale);
     const int threads = 256;
     pack_fields_kernel<<<(cells + threads - 1) / threads, threads, 0, s>>>(
-        ctx->nx, ctx->ny, scale_e, scale_phi, ctx->d_vac, ex, ey, phi, wface, ctx->d_field, ctx->d_barrier);
+        ctx->nx, ctx->ny, tb_closed_edges(ctx), scale_e, scale_phi, ctx->d_vac, ex, ey, phi, wface, ctx->d_field, ctx->d_barrier);
     TB_CUDA(ctx, cudaGetLastError());
     ctx->vscale = vscale;
     ctx->fields_ready = 1;
@@ -1112,6 +1367,7 @@ K32 make_k32(const tb_ctx *ctx, const tb_trace_args *a) {
     k.bytes = tb_halo_count(ctx->nx, ctx->ny) * (int)sizeof(tb_fcell);
     k.pool_off = -1;
     k.reverse = ctx->tune_reverse == 1;
+    k.cell_frame = k.bytes > ctx->smem_attr_bytes;
     k.rec = nullptr;
     k.n_rec = nullptr;
     k.okey = nullptr;
@@ -1124,12 +1380,14 @@ K32 make_k32(const tb_ctx *ctx, const tb_trace_args *a) {
     k.rf_wave = ctx->d_rf_wave;
     k.t_clock = k.t_sec = k.dt_max = k.bvs = k.bvm = 0.f;
     k.short_steps = false;
+    k.wave_scale = 0.f;
     if (a->n_phase > 0) {
         // step time unit dx / vscale: in seconds, in clock units, and the in-flight step bound
         const double unit = ctx->dx / ctx->vscale;
         k.t_sec = (float)unit;
         k.t_clock = (float)(unit / a->period * 4294967296.0);
         k.short_steps = a->dt_max < 0.5 * a->period;
+        k.wave_scale = (float)(a->n_phase * 0x1p-32);
         k.dt_max = (float)(a->dt_max / unit);
         k.bvs = (float)a->bound_vs;
         k.bvm = (float)a->bound_vm;
@@ -1301,10 +1559,10 @@ __device__ __forceinline__ void claim_scatter_body(const K32 &k, int b, int nb) 
             c = claim_class(kk, ion_class);
             int cx, cy;
             float2 u;
-            start_position(x, y, k.inv_dx, k.nx, k.ny, &cx, &cy, &u);
+            start_position(x, y, k.inv_dx, k.nx, k.ny, k.cell_frame, &cx, &cy, &u);
             const float vx = (float)(vx64 * k.inv_v64), vy = (float)(vy64 * k.inv_v64);
-            const float hq = (float)(0.5 * qm64);
-            r0 = make_uint4((unsigned)i, (unsigned)cx | ((unsigned)cy << 16), __float_as_uint(u.x),
+            const float hq = charge_of(qm64, k.cell_frame);
+            r0 = make_uint4((unsigned)i, ((unsigned)cx & 0xffffu) | ((unsigned)cy << 16), __float_as_uint(u.x),
                             __float_as_uint(u.y));
             r1 = make_uint4(__float_as_uint(vx), __float_as_uint(vy), __float_as_uint(hq),
                             (unsigned)n_steps | (sp ? 0x80000000u : 0u));
