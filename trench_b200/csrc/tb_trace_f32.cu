@@ -14,11 +14,11 @@
 //    once per block into shared memory with a bulk async copy (TMA engine,
 //    cp.async.bulk + mbarrier); every bilinear gather is a shared-memory load.  A lane
 //    keeps its quad's corners in registers and loads only when it changes quad.
-//    Grids too large for shared memory, and small batches, read the same layout from
-//    global memory (L2-resident).
-//  * Three forms of a step (field in shared memory).  While every active lane of a warp is in an open quad (no
-//    solid corner, not at the top or bottom edge) the warp runs step_open, which has no
-//    branch; with any lane near a wall it runs step_near, whose extra arithmetic is
+//    Grids too large for shared memory read the same layout from global memory
+//    (L2-resident).
+//  * Three forms of a step (field in shared memory).  While every active lane of a warp is in
+//    an open quad (no solid corner, not at the top or bottom edge) the warp runs step_open,
+//    which has no branch; with any lane near a wall it runs step_near, whose extra arithmetic is
 //    branch-free too; a step that meets a wall, a corner or the edge is not taken there but
 //    left to step_decide, which runs for several such lanes at once.
 //  * Persistent warps, one particle per lane, lanes refill from a global atomic
@@ -464,7 +464,14 @@ __device__ __forceinline__ void cell_step(const K32 &k, const CaseView<false> &C
     const bool escaped = m.niy >= ny;
     bool hit = false, corner = false;
     if (near && !escaped) {
-        hit = !C.F.vac((m.nix + 1) * P + max(m.niy, -1) + 1);
+        if (C.small_steps && s.cy >= 0) {
+            // the end cell is a corner of the quad
+            const bool right = m.dix >= (s.u.x >= 0.5f ? 1 : 0), above = m.niy - s.cy >= (s.u.y >= 0.5f ? 1 : 0);
+            const float f = right ? (above ? q.c11.ex : q.c10.ex) : (above ? q.c01.ex : q.c00.ex);
+            hit = !(__float_as_uint(f) & 1u);
+        } else {
+            hit = !C.F.vac((m.nix + 1) * P + max(m.niy, -1) + 1);
+        }
         // both the column and the (clipped) row changed: a staircase corner may lie on the path
         // between two vacuum cells (trench_charging_2d.py:614-621).  The move reaches the wall
         // only if the cell beyond the first boundary crossed is solid (the first-face rule
@@ -527,6 +534,7 @@ __device__ __forceinline__ void cell_step(const K32 &k, const CaseView<false> &C
         }
     }
     if (!reflected) { s.cx = m.nix; s.cy = m.niy; s.u = m.o; s.v = m.v; }
+    int done = 0;
     if (hit) {
         if (dcell < 0 || dcell >= C.cells) {
             atomicCAS(k.err, TB_DERR_NONE, TB_DERR_BAD_CELL);
@@ -535,13 +543,14 @@ __device__ __forceinline__ void cell_step(const K32 &k, const CaseView<false> &C
         }
         if (a.d_hit) a.d_hit[s.pid] = dcell;
         if (s.spc == 0) ++t.hit_i; else ++t.hit_e;
-        finish_particle<RF>(k, s, t, 1);
+        done = 1;
     } else if (escaped && !reflected) {
         if (s.spc == 0) ++t.esc_i; else ++t.esc_e;
-        finish_particle<RF>(k, s, t, 2);
+        done = 2;
     } else if (s.steps >= s.stop_at) {
-        finish_particle<RF>(k, s, t, 3);
+        done = 3;
     }
+    if (done) finish_particle<RF>(k, s, t, done);
 }
 
 // ---- the vertex frame: fields in shared memory -------------------------------------------
@@ -992,7 +1001,7 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
 
     for (;;) {
         const bool closed = !open && wc >= we;
-        if (closed || __popc(__ballot_sync(FULL, !active)) >= (SMEM ? WAIT_LANES : 1)) {
+        if (closed || __popc(__ballot_sync(FULL, SMEM ? !active : s.pid < 0)) >= (SMEM ? WAIT_LANES : 1)) {
             if constexpr (SMEM) step_held<RF>(k, C, s, t, q, active);
             const unsigned need = __ballot_sync(FULL, s.pid < 0);
             if (closed) {
@@ -1077,21 +1086,19 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
                 }
                 wc = nwc;
                 we = nwe;
-                if (__ballot_sync(FULL, active) == 0u) continue;   // ranks of particles not to be traced
+                if (SMEM && __ballot_sync(FULL, active) == 0u) continue;   // ranks of particles not to be traced
             }
         }
         if constexpr (SMEM) {
             step_warp<RF>(k, C, s, t, q, active, 0x7fffffff,
                           closed ? __popc(__ballot_sync(FULL, active)) : 33 - WAIT_LANES);
-        } else if (__all_sync(FULL, active)) {
+        } else if (__all_sync(FULL, s.pid >= 0)) {
             // step all lanes until a particle ends, one vote per step
             do {
                 cell_step<RF>(k, C, s, t, q);
             } while (__all_sync(FULL, s.pid >= 0));
-            active = s.pid >= 0;
-        } else if (active) {
+        } else if (s.pid >= 0) {
             cell_step<RF>(k, C, s, t, q);
-            active = s.pid >= 0;
         }
     }
 
@@ -1120,13 +1127,12 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
             if (threadIdx.x == 0) s_live = 0;
             if ((int)(threadIdx.x & ~31u) < live) {  // warp-uniform: this warp holds particles
                 int left = TAIL_ROUND_STEPS;
-                while (left > 0 && __any_sync(FULL, active)) {
+                while (left > 0 && __any_sync(FULL, SMEM ? active : s.pid >= 0)) {
                     if constexpr (SMEM) {
                         left -= step_warp<RF>(k, C, s, t, q, active, left, __popc(__ballot_sync(FULL, active)));
                         step_held<RF>(k, C, s, t, q, active);
                     } else {
-                        if (active) cell_step<RF>(k, C, s, t, q);
-                        active = s.pid >= 0;
+                        if (s.pid >= 0) cell_step<RF>(k, C, s, t, q);
                         --left;
                     }
                 }
