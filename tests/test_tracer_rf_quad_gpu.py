@@ -1,0 +1,98 @@
+"""The circuit_rf step that keeps the basis fields with the quad (launches of at most 512
+threads, field in shared memory) against the one that loads them in each step and against FP64.
+
+Both use the same basis values and the same arithmetic, so every launch shape gives the same
+outcomes bit for bit.  The field and basis here are noise from cell to cell, in which an FP32 and
+an FP64 path part after a few hundred steps: the share that ends alike is held to that of the
+FP32 tracer without RF.
+"""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+DX = 5e-9
+PERIOD = 4e-10
+
+
+def mask_of(kind):
+    rng = np.random.default_rng(3)
+    if kind == "posts":
+        vac = rng.random((20, 40)) > 0.12
+        vac[:, 36:] = True
+    elif kind == "one_column":
+        vac = np.ones((1, 30), bool)
+        vac[:, :3] = False
+    else:
+        vac = np.zeros((24, 60), bool)
+        vac[:, 44:] = True
+        vac[8:16, 5:44] = True
+    return vac
+
+
+def trace(vac, n, precision, threads, cfl, n_phase=64):
+    import torch
+    from trench_b200 import _capi
+    from trench_b200.tracer import Context, _ptr
+    L = _capi.lib()
+    rng = np.random.default_rng(17)
+    nx, ny = vac.shape
+    ion = np.arange(n) < n // 2
+    f = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    X = [f(rng.uniform(0, nx * DX, n)), f(np.full(n, (ny - 1e-3) * DX)),
+         f(np.where(ion, rng.normal(0, 2e3, n), rng.normal(0, 7e5, n))),
+         f(-np.where(ion, rng.uniform(5e3, 3e4, n), np.abs(rng.normal(0, 7e5, n)))),
+         f(np.where(ion, 2.4e6, -1.76e11)), f(np.where(ion, 0, 1).astype(np.int8))]
+    EX, EY = (f(a) for a in rng.normal(0, 1e6, (2, nx, ny)))
+    RFX, RFY = (f(a) for a in rng.normal(0, 3e4, (2, 2, nx, ny)))
+    RFP = f(rng.normal(0, 0.05, (2, nx, ny)))
+    WF, PHI = f(np.full((nx, ny), 0.8)), f(rng.normal(0, 2.0, (nx, ny)))
+    t = np.arange(n_phase) / n_phase * 2 * np.pi
+    wave = np.ascontiguousarray(np.stack([30 * np.sin(t), 10 * np.cos(t)], axis=1))
+    WAVE = f(wave)
+    CLOCK = f(np.column_stack((rng.uniform(0, PERIOD, n), np.zeros(n))))
+    ctx = Context(vac, 0, DX)
+    ctx.check(L.tb_set_tuning(ctx.handle, threads, 1))
+    ctx.check(L.tb_set_fields(ctx.handle, _ptr(EX), _ptr(EY), _ptr(PHI), _ptr(WF), 1e5, None))
+    ctx.check(L.tb_set_rf_fields(ctx.handle, _ptr(RFX), _ptr(RFY), _ptr(RFP), _ptr(WF), _ptr(WAVE), n_phase, None))
+    a = _capi.TraceArgs()
+    a.n, a.max_steps, a.step_budget, a.cfl, a.tapered = n, 400, 400, cfl, 1
+    a.d_x, a.d_y, a.d_vx, a.d_vy, a.d_qm, a.d_spc = (_ptr(v) for v in X)
+    a.d_ex, a.d_ey, a.d_phi, a.d_wface = _ptr(EX), _ptr(EY), _ptr(PHI), _ptr(WF)
+    a.d_rf_ex, a.d_rf_ey, a.d_rf_phi, a.d_wave = _ptr(RFX), _ptr(RFY), _ptr(RFP), _ptr(WAVE)
+    a.n_phase, a.period, a.dt_max = n_phase, PERIOD, PERIOD / 8
+    a.bound_vs, a.bound_vm = (float(v) for v in np.abs(wave).max(axis=0))
+    a.d_clock = _ptr(CLOCK)
+    counts = torch.zeros((2, nx, ny), dtype=torch.int32, device="cuda")
+    totals = torch.zeros(8, dtype=torch.int64, device="cuda")
+    status = torch.full((n,), 3, dtype=torch.int8, device="cuda")
+    hit = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+    steps = torch.zeros(n, dtype=torch.int32, device="cuda")
+    a.d_counts, a.d_totals = _ptr(counts), _ptr(totals)
+    a.d_status, a.d_hit, a.d_steps = _ptr(status), _ptr(hit), _ptr(steps)
+    s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    ctx.check(L.tb_trace(ctx.handle, ctypes.byref(a), _capi.PRECISION[precision], s))
+    ctx.check(L.tb_check(ctx.handle, s))
+    out = [v.cpu().numpy() for v in (status, hit, counts, totals)]
+    ctx.close()
+    return out
+
+
+# automatic shape: 128 threads for 4001 particles, 256 for 150,000, 512 for 300,000
+@pytest.mark.parametrize("kind", ["trench", "posts", "one_column"])
+@pytest.mark.parametrize("n,cfl", [(4001, 0.35), (4001, 0.9), (150_000, 0.35), (300_000, 0.35)])
+def test_kept_basis_fields_agree(cuda_device, kind, n, cfl):
+    vac = mask_of(kind)
+    want = trace(vac, n, "f64", 0, cfl)
+    first = None
+    for threads in (0, 256, 1024):
+        status, hit, counts, totals = trace(vac, n, "f32", threads, cfl)
+        same = (status == want[0]) & (hit == want[1])
+        first = first or (status, hit, counts, totals)
+        for a, b in zip(first, (status, hit, counts, totals)):
+            np.testing.assert_array_equal(a, b)
+        assert same.mean() > 0.97
+        assert totals[[0, 1, 2, 4, 5]].sum() == n
+        assert counts.sum() == totals[4] + totals[5]

@@ -214,6 +214,12 @@ __device__ __forceinline__ float charge_of(double qm, bool cell_frame) {
     return cell_frame ? (float)qm : (float)(0.5 * qm);
 }
 
+// Kinds of a circuit_rf step: the basis fields (16 bytes a corner, in global memory) are loaded
+// in each step, or, with the field in shared memory and the registers of at most 512 threads,
+// kept with the quad and loaded ahead of the loop's vote: 1670 -> 1250 us a batch at 512 threads
+// (60 x 250 cells, 2^19 particles).  The 1024-thread kernel (1840 us) would spill them.
+constexpr int RF_STEP = 1, RF_QUAD = 2;
+
 // The four bilinear corners of a lane's quad and their base index (-1 = none).  A step
 // moves under half a cell at the usual CFL, so about half the steps stay in the quad and
 // reload nothing: fewer lanes per gather means fewer shared-memory bank conflicts (or L1
@@ -222,13 +228,27 @@ __device__ __forceinline__ float charge_of(double qm, bool cell_frame) {
 struct QuadCache {
     int base;
     tb_fcell c00, c01, c10, c11;
+    float4 b00, b01, b10, b11;  // circuit_rf, RF_QUAD: the basis fields at the same corners
     // an inactive lane's quad, so that it does not hold its warp up; load() after base = -1 undoes it
     __device__ __forceinline__ void mark_open() { c00.ey = __uint_as_float(__float_as_uint(c00.ey) | 1u); }
     // `last`: the largest base whose four corners lie in the field (a particle with a field
     // or velocity that is not finite may hold any index)
-    template <bool SMEM>
-    __device__ __forceinline__ void load(const FieldView<SMEM> &F, int at, int P, int last) {
+    template <bool SMEM, int RF>
+    __device__ __forceinline__ void load(const FieldView<SMEM> &F, const float4 *rf_field, int at, int P, int last) {
         const int b = SMEM ? (int)min((unsigned)at, (unsigned)last) : at;
+        if (RF == RF_QUAD && SMEM) {
+            asm volatile(
+                "{\n\t.reg .pred c;\n\t"
+                "setp.ne.s32 c, %16, %17;\n\t"
+                "@c ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%18];\n\t"
+                "@c ld.global.nc.v4.f32 {%4, %5, %6, %7}, [%18 + 16];\n\t"
+                "@c ld.global.nc.v4.f32 {%8, %9, %10, %11}, [%19];\n\t"
+                "@c ld.global.nc.v4.f32 {%12, %13, %14, %15}, [%19 + 16];\n\t}"
+                : "+f"(b00.x), "+f"(b00.y), "+f"(b00.z), "+f"(b00.w), "+f"(b01.x), "+f"(b01.y), "+f"(b01.z),
+                  "+f"(b01.w), "+f"(b10.x), "+f"(b10.y), "+f"(b10.z), "+f"(b10.w), "+f"(b11.x), "+f"(b11.y),
+                  "+f"(b11.z), "+f"(b11.w)
+                : "r"(b), "r"(base), "l"(rf_field + b), "l"(rf_field + b + P));
+        }
         if (SMEM) {
             // predicated in place: a branch around the loads costs more than the loads
             const uint32_t a0 = F.shared_address() + 8u * (unsigned)b, a1 = a0 + 8u * (unsigned)P;
@@ -306,7 +326,7 @@ __device__ __forceinline__ double wrap_column(double x, int nx) {
 
 // Writes the outputs of a particle that is absorbed (1), escaped (2) or stopped at its step
 // cap (3) and empties the lane.
-template <bool RF>
+template <int RF>
 __device__ __forceinline__ void finish_particle(const K32 &k, LaneState &s, LaneTally &t, int done) {
     const tb_trace_args &a = k.a;
     const int pid = s.pid;
@@ -331,11 +351,11 @@ __device__ __forceinline__ void finish_particle(const K32 &k, LaneState &s, Lane
 }
 
 // Quad of a particle: its vertex, or in the cell frame the vertex nearest to its offset.
-template <bool SMEM>
-__device__ __forceinline__ void load_quad(const CaseView<SMEM> &C, const LaneState &s, QuadCache &q) {
+template <bool SMEM, int RF>
+__device__ __forceinline__ void load_quad(const K32 &k, const CaseView<SMEM> &C, const LaneState &s, QuadCache &q) {
     int at = s.cx * C.P + s.cy;
     if (!SMEM) at = (s.cx + (s.u.x >= 0.5f ? 1 : 0)) * C.P + max(s.cy + (s.u.y >= 0.5f ? 1 : 0), 0);
-    q.load(C.F, at, C.P, C.last);
+    q.template load<SMEM, RF>(C.F, k.rf_field, at, C.P, C.last);
 }
 
 // ---- the cell frame: fields in global memory ---------------------------------------------
@@ -349,7 +369,7 @@ __device__ __forceinline__ int cell_rf_interval(const K32 &k, uint32_t clock, fl
 }
 
 // Acceleration A, time step and clock advance of the next step (see step_size).
-template <bool RF>
+template <int RF>
 __device__ __forceinline__ void cell_step_size(const K32 &k, const CaseView<false> &C, const LaneState &s,
                                                const QuadCache &q, bool near, float2 &A, float &dt, uint32_t &inc) {
     const float2 tq = __fadd2_rn(s.u, make_float2(s.u.x >= 0.5f ? -0.5f : 0.5f, s.u.y >= 0.5f ? -0.5f : 0.5f));
@@ -443,12 +463,12 @@ __device__ __forceinline__ CellMove cell_move(const CaseView<false> &C, const La
 // One step of one particle (trench_charging_2d.py:584-650), as step_open and step_decide
 // together; these steps wait for the field's loads, and one branch a step costs less than the
 // lanes that three forms hold back.
-template <bool RF>
+template <int RF>
 __device__ __forceinline__ void cell_step(const K32 &k, const CaseView<false> &C, LaneState &s, LaneTally &t,
                                           QuadCache &q) {
     const tb_trace_args &a = k.a;
     const int ny = C.ny, P = C.P;
-    load_quad(C, s, q);
+    load_quad<false, RF>(k, C, s, q);
     // a step below half a cell ends in a corner cell of its quad
     const bool near = !(C.small_steps && is_open(q.c00));
     float2 A;
@@ -559,7 +579,7 @@ __device__ __forceinline__ void cell_step(const K32 &k, const CaseView<false> &C
 // (trench_charging_2d.py:492-509, 587-608): vacuum-weighted bilinear field and the CFL step
 // dt = cfl / (|v| + sqrt(2 |a|) + 1 m/s), with sqrt(2 |a|) = 2 (|h|^2)^(1/4).  NEAR: the quad may
 // hold solid corners, whose weights are left out; otherwise the vacuum weights sum to one.
-template <bool RF, bool NEAR>
+template <int RF, bool NEAR>
 __device__ __forceinline__ void step_size(const K32 &k, const CaseView<true> &C, const LaneState &s,
                                           const QuadCache &q, float2 &h, float &dt, uint32_t &inc) {
     const float tx = s.u.x + 0.5f, ty = s.u.y + 0.5f;
@@ -591,8 +611,11 @@ __device__ __forceinline__ void step_size(const K32 &k, const CaseView<true> &C,
         float w0;
         const int i0 = rf_interval(k, c0, w0);
         const float4 e0 = __ldg(k.rf_wave + i0);
-        const float4 b00 = __ldg(k.rf_field + base), b01 = __ldg(k.rf_field + base + 1);
-        const float4 b10 = __ldg(k.rf_field + base + P), b11 = __ldg(k.rf_field + base + P + 1);
+        float4 b00 = q.b00, b01 = q.b01, b10 = q.b10, b11 = q.b11;
+        if (RF == RF_STEP) {
+            b00 = __ldg(k.rf_field + base); b01 = __ldg(k.rf_field + base + 1);
+            b10 = __ldg(k.rf_field + base + P); b11 = __ldg(k.rf_field + base + P + 1);
+        }
         const float2 Es = bilinear2(make_float2(b00.x, b00.y), make_float2(b01.x, b01.y), make_float2(b10.x, b10.y),
                                     make_float2(b11.x, b11.y), txx, tyy);
         const float2 Em = bilinear2(make_float2(b00.z, b00.w), make_float2(b01.z, b01.w), make_float2(b10.z, b10.w),
@@ -638,7 +661,7 @@ __device__ __forceinline__ int wrap_vertex(int c, int nx) {
 }
 
 // Takes a step of length dt to offset p (r = rounded(p)) from the present vertex.
-template <bool RF>
+template <int RF>
 __device__ __forceinline__ void take_step(const K32 &k, const CaseView<true> &C, LaneState &s, QuadCache &q, float2 h,
                                           float dt, uint32_t inc, float2 p, float2 r) {
     const float d2 = dt + dt;
@@ -650,14 +673,14 @@ __device__ __forceinline__ void take_step(const K32 &k, const CaseView<true> &C,
         s.clock += inc;
         s.elapsed += dt * k.t_sec;
     }
-    load_quad(C, s, q);
+    load_quad<true, RF>(k, C, s, q);
 }
 
 // A step of a warp whose lanes' quads are all open: a step moves at most cfl cells (|v| dt +
 // |a| dt^2 / 2 <= cfl for the CFL dt), so with cfl below one half it ends in one of the quad's
 // four corner cells, all vacuum.  Inactive lanes take a step of length zero, which leaves them
 // exactly as they are.
-template <bool RF>
+template <int RF>
 __device__ __forceinline__ void step_open(const K32 &k, const CaseView<true> &C, LaneState &s, QuadCache &q,
                                           bool active) {
     float2 h;
@@ -675,7 +698,7 @@ __device__ __forceinline__ void step_open(const K32 &k, const CaseView<true> &C,
 // A step of a warp with lanes near a wall or an edge of the grid.  It is taken if it ends in a
 // vacuum cell of the grid with no staircase corner on the way; otherwise the particle stays as
 // it was and the return is false: the step needs the decisions of step_decide.
-template <bool RF>
+template <int RF>
 __device__ __forceinline__ bool step_near(const K32 &k, const CaseView<true> &C, LaneState &s, QuadCache &q,
                                           bool active) {
     float2 h;
@@ -714,7 +737,7 @@ __device__ __forceinline__ bool step_near(const K32 &k, const CaseView<true> &C,
 // One step of one particle with everything it may meet (trench_charging_2d.py:584-650):
 // escape, staircase corner, first-face wall entry, barrier reflection, the step cap (s.steps
 // counts the step already); an ended particle's outputs are written and s.pid becomes -1.
-template <bool RF>
+template <int RF>
 __device__ __forceinline__ void step_decide(const K32 &k, const CaseView<true> &C, LaneState &s, LaneTally &t,
                                             QuadCache &q) {
     const int nx = C.nx, ny = C.ny, P = C.P;
@@ -812,7 +835,7 @@ __device__ __forceinline__ void step_decide(const K32 &k, const CaseView<true> &
             s.clock += inc;
             s.elapsed += dt * k.t_sec;
         }
-        load_quad(C, s, q);
+        load_quad<true, RF>(k, C, s, q);
     }
 
     if (hit) {
@@ -840,7 +863,7 @@ constexpr int POOL_WORDS = 9;
 constexpr int POOL_WORDS_RF = 11;   // + phase, elapsed
 constexpr int TAIL_ROUND_STEPS = 64;
 
-template <bool RF>
+template <int RF>
 __device__ __forceinline__ void pool_put(uint32_t *P, int T, int q, const LaneState &s) {
     P[0 * T + q] = (uint32_t)s.pid;
     P[1 * T + q] = ((uint32_t)s.cx & 0xffffu) | ((uint32_t)s.cy << 16);
@@ -857,7 +880,7 @@ __device__ __forceinline__ void pool_put(uint32_t *P, int T, int q, const LaneSt
     }
 }
 
-template <bool RF>
+template <int RF>
 __device__ __forceinline__ void pool_get(const uint32_t *P, int T, int q, LaneState &s) {
     s.pid = (int)P[0 * T + q];
     const uint32_t xy = P[1 * T + q];
@@ -883,7 +906,7 @@ __device__ __forceinline__ void pool_get(const uint32_t *P, int T, int q, LaneSt
 // after `limit` steps; particles at their cap end here.  Returns the steps made.  Every lane
 // of the warp calls it.  While every active lane's quad is open the whole warp runs step_open,
 // which has no branch; the cached quad of an inactive lane is marked open.
-template <bool RF>
+template <int RF>
 __device__ __forceinline__ int step_warp(const K32 &k, const CaseView<true> &C, LaneState &s, LaneTally &t,
                                          QuadCache &q, bool &active, int limit, int least) {
     const unsigned FULL = 0xffffffffu;
@@ -915,7 +938,7 @@ __device__ __forceinline__ int step_warp(const K32 &k, const CaseView<true> &C, 
 }
 
 // The decision steps of the held lanes (occupied, not active).
-template <bool RF>
+template <int RF>
 __device__ __forceinline__ void step_held(const K32 &k, const CaseView<true> &C, LaneState &s, LaneTally &t,
                                           QuadCache &q, bool &active) {
     if (s.pid >= 0 && !active) {
@@ -926,7 +949,7 @@ __device__ __forceinline__ void step_held(const K32 &k, const CaseView<true> &C,
             s.cy = 0;
         }
         q.base = -1;
-        load_quad(C, s, q);
+        load_quad<true, RF>(k, C, s, q);
         ++s.steps;
         step_decide<RF>(k, C, s, t, q);
         active = s.pid >= 0;
@@ -954,7 +977,7 @@ constexpr int WAIT_LANES = 6;
 // rounds: the live particles are packed into the first warps, those warps take up
 // to TAIL_ROUND_STEPS steps, and the rest wait at the barrier.  A particle's
 // arithmetic does not depend on its lane, so the results are the same either way.
-template <bool SMEM, bool RF, bool REC = false>
+template <bool SMEM, int RF, bool REC = false>
 __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, uint32_t *pool) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -985,7 +1008,8 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
     QuadCache q;          // always a quad of the grid: an inactive lane reads its fields too
     q.base = -1;
     q.c00 = q.c01 = q.c10 = q.c11 = tb_fcell{0.f, 0.f};
-    q.load(C.F, 0, C.P, C.last);
+    q.b00 = q.b01 = q.b10 = q.b11 = make_float4(0.f, 0.f, 0.f, 0.f);
+    q.template load<SMEM, RF>(C.F, k.rf_field, 0, C.P, C.last);
     q.mark_open();
     bool active = false;   // the lane holds a particle that is not waiting for a decision step
     bool open = true;
@@ -1082,7 +1106,7 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
                     }
                     active = s.pid >= 0;
                     q.base = -1;
-                    if (SMEM && active) load_quad(C, s, q);
+                    if (SMEM && active) load_quad<SMEM, RF>(k, C, s, q);
                 }
                 wc = nwc;
                 we = nwe;
@@ -1118,7 +1142,7 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
             if ((int)threadIdx.x < live) {
                 pool_get<RF>(pool, T, threadIdx.x, s);
                 q.base = -1;
-                if (SMEM) load_quad(C, s, q);
+                if (SMEM) load_quad<SMEM, RF>(k, C, s, q);
             } else if (SMEM) {
                 q.mark_open();
             }
@@ -1173,7 +1197,7 @@ __global__ void __launch_bounds__(THREADS, 1) trace_f32_kernel(const __grid_cons
         fieldp = reinterpret_cast<const tb_fcell *>(smem_raw);
     }
     uint32_t *pool = k.pool_off >= 0 ? reinterpret_cast<uint32_t *>(smem_raw + k.pool_off) : nullptr;
-    run_case<SMEM, RF, REC>(k, fieldp, pool);
+    run_case<SMEM, RF ? (SMEM && THREADS <= 512 ? RF_QUAD : RF_STEP) : 0, REC>(k, fieldp, pool);
 }
 
 // Many cases in one persistent launch: each CTA repeatedly takes the case with the
@@ -1222,9 +1246,9 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
             fieldp = reinterpret_cast<const tb_fcell *>(smem_raw);
         }
         uint32_t *pool = k.pool_off >= 0 ? reinterpret_cast<uint32_t *>(smem_raw + k.pool_off) : nullptr;
-        if (k.a.n_phase > 0) run_case<SMEM, true>(k, fieldp, pool);  // block-uniform: one case per CTA
-        else if (SMEM && k.rec) run_case<SMEM, false, SMEM>(k, fieldp, pool);
-        else run_case<SMEM, false>(k, fieldp, pool);
+        if (k.a.n_phase > 0) run_case<SMEM, RF_STEP>(k, fieldp, pool);  // block-uniform: one case per CTA
+        else if (SMEM && k.rec) run_case<SMEM, 0, SMEM>(k, fieldp, pool);
+        else run_case<SMEM, 0>(k, fieldp, pool);
         __syncthreads();  // every warp is done with this case's field
     }
 }
@@ -1752,6 +1776,11 @@ int tb_launch_trace_f32(tb_ctx *ctx, const tb_trace_args *a, cudaStream_t s) {
         // by batch size: the largest CTA that still puts one on every SM
         const long long per_sm_n = (a->n + ctx->num_sms - 1) / std::max(ctx->num_sms, 1);
         threads = per_sm_n >= 768 ? 1024 : per_sm_n >= 384 ? 512 : per_sm_n >= 192 ? 256 : 128;
+        // circuit_rf with the field in shared memory: at most 512 threads, whose registers hold
+        // the basis fields of a quad.  60 x 250 cells, us a batch at 128, 256, 512 and 1024
+        // threads: 734, 765, 809, 1093 (405 particles per SM), 925, 844, 901, 1077 (811), 1492, 1030,
+        // 1037, 1238 (1771), 2684, 1695, 1253, 1839 (3542), 5131, 3021, 2072, 3393 (7085).
+        if (rf && smem) threads = per_sm_n >= 1536 ? 512 : per_sm_n >= 512 ? 256 : 128;
     }
     // the drain pool goes after the field when both fit (without the field it always fits
     // under the default 48 KB)
