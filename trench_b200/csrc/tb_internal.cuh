@@ -100,7 +100,7 @@ __device__ __forceinline__ void tb_store_packed(tb_fcell *out, const uint8_t *va
 
 struct tb_ctx;
 // Whether the packed field's edge quads are left unflagged: the shared-memory tracer takes the flag
-// for "open", the global-memory one looks at the row.
+// for "no step leaves the grid" too, the global-memory one tests every step's end row.
 inline bool tb_closed_edges(const tb_ctx *ctx);
 
 struct tb_poisson;
