@@ -77,10 +77,9 @@ __device__ __forceinline__ void tb_store_halo(T *out, int nx, int ny, int ix, in
 }
 
 // tb_store_halo for the packed tracer field: every padded copy of cell (ix, iy) gets the
-// quad flag of its own padded position in bit 0 of ey; with `edges` the quads of the top and
-// bottom halo rows, where a step may leave the grid, are not flagged (tb_closed_edges).
+// quad flag of its own padded position in bit 0 of ey.
 __device__ __forceinline__ void tb_store_packed(tb_fcell *out, const uint8_t *vac, int nx, int ny, int ix, int iy,
-                                                bool edges, tb_fcell v) {
+                                                tb_fcell v) {
     const int P = ny + 2;
     int cs[3], rs[3], nc = 0, nr = 0;
     cs[nc++] = ix + 1;
@@ -92,16 +91,10 @@ __device__ __forceinline__ void tb_store_packed(tb_fcell *out, const uint8_t *va
     const uint32_t by = __float_as_uint(v.ey) & ~1u;
     for (int a = 0; a < nc; ++a)
         for (int b = 0; b < nr; ++b) {
-            const bool edge = rs[b] == 0 || rs[b] >= ny;
-            const uint32_t q = !(edges && edge) && tb_quad_vacuum(vac, nx, ny, cs[a], rs[b]) ? 1u : 0u;
+            const uint32_t q = tb_quad_vacuum(vac, nx, ny, cs[a], rs[b]) ? 1u : 0u;
             out[cs[a] * P + rs[b]] = tb_fcell{v.ex, __uint_as_float(by | q)};
         }
 }
-
-struct tb_ctx;
-// Whether the packed field's edge quads are left unflagged: the shared-memory tracer takes the flag
-// for "no step leaves the grid" too, the global-memory one tests every step's end row.
-inline bool tb_closed_edges(const tb_ctx *ctx);
 
 struct tb_poisson;
 void tb_poisson_free(tb_poisson *ps);
@@ -162,10 +155,6 @@ int tb_cuda_check(tb_ctx *ctx, cudaError_t e, const char *what);
         if (e_ != cudaSuccess) return tb_cuda_check(ctx, e_, #call); \
     } while (0)
 
-inline bool tb_closed_edges(const tb_ctx *ctx) {
-    return tb_halo_count(ctx->nx, ctx->ny) * (int)sizeof(tb_fcell) <= ctx->smem_attr_bytes;
-}
-
 // Launchers implemented per translation unit.
 int tb_launch_trace_f64(tb_ctx *ctx, const tb_trace_args *a, cudaStream_t s);
 int tb_launch_trace_f32(tb_ctx *ctx, const tb_trace_args *a, cudaStream_t s);
@@ -180,7 +169,6 @@ int tb_launch_pack_rf_fields(tb_ctx *ctx, const double *rf_ex, const double *rf_
 struct tb_pack_step_entry {
     tb_step_desc d;
     int nx, ny;
-    bool edges;
     const uint8_t *vac;
     double scale_e, scale_phi;
     tb_fcell *field;

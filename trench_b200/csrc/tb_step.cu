@@ -305,7 +305,7 @@ __global__ void k_monitors(const tb_step_desc d, const double *w, const uint8_t 
 
 // K5: E = -grad phi over vacuum neighbours (trench_charging_2d.py:429-454), the
 // packed FP32 tracer field, the per-face wall barrier and the probe history.
-__device__ __forceinline__ void field_cell(const tb_step_desc &d, int c, int nx, int ny, bool edges, const uint8_t *vac,
+__device__ __forceinline__ void field_cell(const tb_step_desc &d, int c, int nx, int ny, const uint8_t *vac,
                                            double scale_e, double scale_phi, tb_fcell *out, float4 *bar) {
     const int n = nx * ny;
     if (c == 0) {
@@ -342,7 +342,7 @@ __device__ __forceinline__ void field_cell(const tb_step_desc &d, int c, int nx,
     const double ex = -gx, ey = -gy;
     if (d.d_ex) { d.d_ex[c] = ex; d.d_ey[c] = ey; }
     const int v = vac[c] ? 1 : 0;
-    tb_store_packed(out, vac, nx, ny, ix, iy, edges, tb_pack_cell(ex, ey, v, scale_e));
+    tb_store_packed(out, vac, nx, ny, ix, iy, tb_pack_cell(ex, ey, v, scale_e));
     float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
     if (!v && d.d_wface) {
         const double f = d.d_wface[c];
@@ -354,9 +354,9 @@ __device__ __forceinline__ void field_cell(const tb_step_desc &d, int c, int nx,
     bar[c] = b;
 }
 
-__global__ void k_field(const tb_step_desc d, int nx, int ny, bool edges, const uint8_t *vac, double scale_e, double scale_phi,
+__global__ void k_field(const tb_step_desc d, int nx, int ny, const uint8_t *vac, double scale_e, double scale_phi,
                         tb_fcell *out, float4 *bar) {
-    field_cell(d, blockIdx.x * blockDim.x + threadIdx.x, nx, ny, edges, vac, scale_e, scale_phi, out, bar);
+    field_cell(d, blockIdx.x * blockDim.x + threadIdx.x, nx, ny, vac, scale_e, scale_phi, out, bar);
 }
 
 // ---- the same update for every case of a pack, one launch per stage ----------------
@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(PACK_THREADS) k_pack_green(const tb_pack_step_
 
 __global__ void __launch_bounds__(PACK_THREADS) k_pack_field(const tb_pack_step_entry *E) {
     const tb_pack_step_entry &e = E[blockIdx.y];
-    field_cell(e.d, blockIdx.x * blockDim.x + threadIdx.x, e.nx, e.ny, e.edges, e.vac, e.scale_e, e.scale_phi, e.field,
+    field_cell(e.d, blockIdx.x * blockDim.x + threadIdx.x, e.nx, e.ny, e.vac, e.scale_e, e.scale_phi, e.field,
                e.bar);
 }
 
@@ -434,7 +434,7 @@ extern "C" int tb_step_potential(tb_ctx *ctx, const tb_step_desc *d, void *strea
                                                   d->d_rows);
     const int cells = ctx->nx * ctx->ny;
     const double scale_e = ctx->dx / (d->vscale * d->vscale), scale_phi = 1.0 / (d->vscale * d->vscale);
-    k_field<<<(cells + 255) / 256, 256, 0, s>>>(*d, ctx->nx, ctx->ny, tb_closed_edges(ctx), ctx->d_vac, scale_e, scale_phi, ctx->d_field,
+    k_field<<<(cells + 255) / 256, 256, 0, s>>>(*d, ctx->nx, ctx->ny, ctx->d_vac, scale_e, scale_phi, ctx->d_field,
                                                ctx->d_barrier);
     TB_CUDA(ctx, cudaGetLastError());
     ctx->vscale = d->vscale;
@@ -536,7 +536,6 @@ int tb_pack_steps_set(tb_pack_steps **out, int n, tb_ctx *const *ctxs, const tb_
         e.d = d;
         e.nx = c->nx;
         e.ny = c->ny;
-        e.edges = tb_closed_edges(c);
         e.vac = c->d_vac;
         e.scale_e = c->dx / (d.vscale * d.vscale);
         e.scale_phi = 1.0 / (d.vscale * d.vscale);

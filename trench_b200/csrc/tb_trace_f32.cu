@@ -4,10 +4,12 @@
 // roots are the hardware approximations (max 2 ulp), denormals flush to zero (the
 // vacuum flag stored in the low bit of a zero field is such a denormal).
 // Design (B200-first):
-//  * Position = nearest grid vertex (integers) + FP32 offset in [-0.5, 0.5] cells, so the
-//    index and the periodic wrap are exact integer operations, the offset keeps 2^-25-cell
-//    resolution everywhere in the grid, and the vertex is the index of the bilinear quad.
-//    With the field in global memory: cell + offset in [0, 1) (see LaneState).
+//  * Position = integer cell + FP32 offset in [0,1) cell units, so the cell
+//    index, periodic wrap and floor are exact integer operations and the offset
+//    keeps 2^-24-cell resolution everywhere in the grid and below it.
+//  * One arithmetic: every form of a step, with the field in shared or global memory, takes
+//    its quad, step length and move from the same functions, whose roundings the compiler cannot
+//    change, so a particle ends the same whatever launch, form or lane steps it.
 //  * Velocities in units of vscale (m/s); time in dx/vscale; the packed field is
 //    E*vac*dx/vscale^2 so qm*field is the acceleration in these units.
 //  * The packed field (8 bytes per cell, vacuum flag in bit 0 of Ex) is staged
@@ -17,14 +19,16 @@
 //    Grids too large for shared memory read the same layout from global memory
 //    (L2-resident).
 //  * Three forms of a step (field in shared memory).  While every active lane of a warp is in
-//    an open quad (no solid corner, not at the top or bottom edge) the warp runs step_open,
-//    which has no branch; with any lane near a wall it runs step_near, whose extra arithmetic is
-//    branch-free too; a step that meets a wall, a corner or the edge is not taken there but
-//    left to step_decide, which runs for several such lanes at once.
-//  * Persistent warps, one particle per lane, lanes refill from a global atomic
-//    queue as soon as their particle ends (no lane waits for a slow electron); a warp
-//    reserves a small block of ranks at a time and prefetches their particles into
-//    L1, so most refills wait neither for the atomic nor for the particle's loads.
+//    an open quad (no solid corner, not at the top edge) the warp runs step_open, which has no
+//    branch; with any lane near a wall it runs step_near, whose extra arithmetic is branch-free
+//    too; a step that meets a wall, a corner or the edge is not taken there but left to
+//    step_full, which runs for several such lanes at once.  Fields in global memory take every
+//    step in step_full.
+//  * Persistent warps, one particle per lane.  Lanes whose particle has ended refill from a
+//    global atomic queue: at once with the field in global memory, and once WAIT_LANES of a warp
+//    wait with it in shared memory.  A warp reserves a small block of ranks at a time and
+//    prefetches their particles into L1, so most refills wait neither for the atomic nor for
+//    the particle's loads.
 //  * Claim order (tb_set_claim_order): index, reverse, or learned -- electrons first,
 //    then ions longest predicted first from per-bin step means of the previous trace,
 //    claimed through FP32 claim records written in that order by a scatter kernel.
@@ -32,12 +36,12 @@
 //  * The x/y-symmetric arithmetic of a step (the bilinear sums of (Ex, Ey), acceleration,
 //    velocity and position updates, rounding to the vertex) runs on packed FP32 pairs
 //    (sm_100 f32x2 add/mul/fma): one instruction per pair.
-// What bounds it: instruction issue.  Open space (an all-vacuum 60 x 200 grid, 2.4M
-// particles): 69.9 warp instructions and 80 cycles per scheduler and warp-step, 87 % of the
-// issue slots (before the vertex frame, the cached quads and the three forms: 87.9
-// instructions, 107 cycles; without the cached quads the gathers' bank conflicts, 24 shared-
-// memory wavefronts a warp-step, held it at 102).  AR-8 trench, 2^20 particles: 1.257 ms
-// against 1.416 ms a launch; walls are near some lane in 45 % of the warp-steps.
+// What bounds it: instruction issue with the field in shared memory (without the cached quads also
+// the gathers' bank conflicts), one particle's chain of dependent steps in small batches, the
+// gathers' latency with the field in global memory.  Whole batches, one form of a step and no
+// cached quads -> three forms with them: 60 x 200 cells, 6000 particles 893 -> 689 us; 60 x 250
+// cells, 2^20 particles 1728 -> 1613 us, untapered 2^22 particles 4095 -> 3998 us; 8 uneven cases in
+// one launch 3185 -> 2680 us.
 // The step follows the reference algorithm (trench_charging_2d.py:584-650,
 // trench_trace.cu:92-148): vacuum-weighted bilinear field, CFL step, trapezoid
 // update, periodic x, escape at the top, staircase corner crossing, first-face
@@ -64,7 +68,6 @@ struct K32 {
     int bytes;                      // packed field bytes (multiple of 16)
     int pool_off;                   // byte offset of the drain pool in dynamic shared memory, -1 = none
     int reverse;                    // claim particles from the last index down
-    bool cell_frame;                // claim records hold cell and offset (see LaneState)
     // learned claim order (nullptr rec = none): claim records in claim order, their number,
     // each particle's key, the ion bins' classes, per-block class starts, per-bin step sums,
     // 1 / domain width and the ordering kernels' blocks
@@ -85,7 +88,8 @@ struct K32 {
     const float4 *rf_wave;          // (vs_i, vm_i, vs_i+1 - vs_i, vm_i+1 - vm_i), i < n_phase
     float t_clock;                  // clock units (2^-32 period) per unit of step time
     bool short_steps;               // every step is under half a period (clock steps fit 32 bits)
-    float wave_scale;               // n_phase * 2^-32: clock -> table position (cell frame)
+    float minus_zero;               // -0 (see move_by)
+    float wave_scale;               // n_phase * 2^-32: clock -> table position
     float t_sec;                    // seconds per unit of step time (dx / vscale)
     float dt_max;                   // step bound of the in-flight field, in step time
     float bvs, bvm;                 // largest voltage deltas of the waveform
@@ -150,92 +154,55 @@ __device__ bool stage_field(void *dst, const void *src, int bytes, uint64_t *mba
     return __syncthreads_and(done) != 0;
 }
 
-// One lane's particle.  The position is held relative to the nearest grid vertex: vertex
-// (cx, cy) is the corner shared by padded cells (cx, cy) .. (cx + 1, cy + 1), so it is also the
-// index of the bilinear quad the particle interpolates from, and u in [-0.5, 0.5] is the offset
-// from it in cells (two bits finer than an offset in [0, 1), and tx = u + 0.5 needs no selects).
-// cx in [0, nx] (0 and nx are the same vertex), cy in [0, ny]; a particle below the grid (open
-// bottom rows only) has cy = 0 and the rest of its distance in u.y.  Velocity in vscale units;
-// hq is half the charge-to-mass ratio.  pid < 0 = no particle.
-// Fields in global memory (SMEM = false): the cell frame -- cx, cy is the particle's cell (cy < 0
-// below the grid), u in [0, 1) its offset in it, hq the whole charge-to-mass ratio.  The vertex
-// frame and its three forms of a step measured 2650 against 3150 us a batch there (200 x 700
-// cells, 2^19 particles), with as many particles that end elsewhere than in FP64 (163 and 158 of
-// 3.1e6), but not the same ones: on so fine a grid each one moves the batch's potential by
-// more than batches may differ.
+// One lane's particle: cell (ix, iy) and FP32 offset o in [0, 1) from its lower-left corner, in
+// cells (below the grid, through open bottom rows only, iy is negative); velocity in vscale units;
+// pid < 0 = no particle.
 struct LaneState {
-    int pid, cx, cy, steps, stop_at, spc;
-    float2 u, v;                    // offset and velocity, packed pairs
-    float hq;
+    int pid, ix, iy, steps, stop_at, spc;
+    float2 o, v;                    // offset and velocity, packed pairs
+    float qm;
     uint32_t clock;                 // circuit_rf: clock in 2^-32 of the period
     float elapsed;                  // circuit_rf: seconds in flight
 };
 
-// Adding MAGIC (1.5 x 2^23) to a value below 2^22 rounds it to the nearest integer, which the
-// low mantissa bits then hold: as_int(x + MAGIC) - MAGIC_BITS.  Nearest-vertex indices come
-// from this instead of floor and float-to-int conversions (both on the conversion pipe, at a
-// quarter of the packed-add rate).
-constexpr float MAGIC = 12582912.f;
-constexpr int MAGIC_BITS = 0x4b400000;
-
-// Vertex and offset of a coordinate in cells, clamped into a grid of n cells; the row keeps
-// the distance below the grid in the offset (see LaneState).
-__device__ __forceinline__ void vertex_of(double xc, int cell, int *c, float *u) {
-    const double d = fmin(fmax(xc - (double)cell, 0.0), 1.0 - 0x1p-24);
-    const int h = d >= 0.5 ? 1 : 0;
-    *c = cell + h;
-    *u = (float)(d - (double)h);
-}
 constexpr float ONE_BELOW = 0x1.fffffep-1f;  // largest float < 1
-__device__ __forceinline__ void start_position(const double x, const double y, double inv_dx, int nx, int ny,
-                                               bool cell_frame, int *cx, int *cy, float2 *u) {
-    // x lies in cell min(int(x/dx), nx-1) as in the reference (trench_charging_2d.py:611); a
-    // start above the grid escapes at once
+
+// Cell and offset of a start position in metres.  x lies in cell min(int(x/dx), nx-1) as in the
+// reference (trench_charging_2d.py:611); a start above the grid is put at the grid's top.
+__device__ __forceinline__ void start_position(const double x, const double y, double inv_dx, int nx, int ny, int &ix,
+                                               int &iy, float2 &o) {
     const double xc = x * inv_dx, yc = y * inv_dx;
-    const int ix = min(max((int)xc, 0), nx - 1);
-    if (cell_frame) {
-        const int iy = min((int)floor(yc), ny - 1);
-        *cx = ix;
-        *cy = iy;
-        u->x = fminf(fmaxf((float)(xc - (double)ix), 0.f), ONE_BELOW);
-        u->y = fminf(fmaxf((float)(yc - (double)iy), 0.f), ONE_BELOW);
-        return;
-    }
-    vertex_of(xc, ix, cx, &u->x);
-    if (yc < 0.0) {
-        *cy = 0;
-        u->y = (float)fmax(yc, -1e6);
-    } else {
-        vertex_of(yc, min((int)yc, ny - 1), cy, &u->y);
-    }
-}
-// Half the charge-to-mass ratio (vertex frame) or all of it (cell frame).
-__device__ __forceinline__ float charge_of(double qm, bool cell_frame) {
-    return cell_frame ? (float)qm : (float)(0.5 * qm);
+    ix = min(max((int)xc, 0), nx - 1);
+    iy = min((int)floor(yc), ny - 1);
+    o.x = fminf(fmaxf((float)(xc - (double)ix), 0.f), ONE_BELOW);
+    o.y = fminf(fmaxf((float)(yc - (double)iy), 0.f), ONE_BELOW);
 }
 
 // Kinds of a circuit_rf step: the basis fields (16 bytes a corner, in global memory) are loaded
 // in each step, or, with the field in shared memory and the registers of at most 512 threads,
-// kept with the quad and loaded ahead of the loop's vote: 1670 -> 1250 us a batch at 512 threads
-// (60 x 250 cells, 2^19 particles).  The 1024-thread kernel (1840 us) would spill them.
+// kept with the quad and loaded ahead of the loop's vote.  The 1024-thread kernel would spill them.
 constexpr int RF_STEP = 1, RF_QUAD = 2;
 
 // The four bilinear corners of a lane's quad and their base index (-1 = none).  A step
 // moves under half a cell at the usual CFL, so about half the steps stay in the quad and
 // reload nothing: fewer lanes per gather means fewer shared-memory bank conflicts (or L1
-// lines).  The corners of the next quad are loaded at the end of a step, ahead of the
-// loop's vote.
+// lines).  With the field in shared memory the corners of the next quad are loaded at the end
+// of a step, ahead of the loop's vote.
 struct QuadCache {
     int base;
+    int row;                    // padded row of the lower corners, before its clamp at the bottom
+    float2 t;                   // the particle's position between the corners, in [0, 1)
     tb_fcell c00, c01, c10, c11;
-    float4 b00, b01, b10, b11;  // circuit_rf, RF_QUAD: the basis fields at the same corners
-    // an inactive lane's quad, so that it does not hold its warp up; load() after base = -1 undoes it
-    __device__ __forceinline__ void mark_open() { c00.ey = __uint_as_float(__float_as_uint(c00.ey) | 1u); }
-    // `last`: the largest base whose four corners lie in the field (a particle with a field
-    // or velocity that is not finite may hold any index)
+    float4 b00, b01, b10, b11;  // circuit_rf: the basis fields at the same corners
+    __device__ __forceinline__ void load_basis(const float4 *rf_field, int P) {
+        b00 = __ldg(rf_field + base); b01 = __ldg(rf_field + base + 1);
+        b10 = __ldg(rf_field + base + P); b11 = __ldg(rf_field + base + P + 1);
+    }
+    // `last`: the largest base whose four corners lie in the field (circuit_rf: a step of dt_max
+    // from rest in a field below FP32's squares, or of one that is not a number, may leave the grid)
     template <bool SMEM, int RF>
     __device__ __forceinline__ void load(const FieldView<SMEM> &F, const float4 *rf_field, int at, int P, int last) {
-        const int b = SMEM ? (int)min((unsigned)at, (unsigned)last) : at;
+        const int b = SMEM && RF ? (int)min((unsigned)at, (unsigned)last) : at;
         if (RF == RF_QUAD && SMEM) {
             asm volatile(
                 "{\n\t.reg .pred c;\n\t"
@@ -277,8 +244,7 @@ struct LaneTally {
     unsigned steps, esc_i, esc_e, lost, hit_i, hit_e;
 };
 
-// The quad flag of a quad's lower-left corner (tb_quad_vacuum): all four cells vacuum and, in
-// shared memory, no step leaves the grid.
+// The quad flag of a quad's lower-left corner (tb_quad_vacuum): all four cells vacuum.
 __device__ __forceinline__ bool is_open(const tb_fcell &c00) { return __float_as_uint(c00.ey) & 1u; }
 
 // Loop-invariant parameters of one case.
@@ -289,39 +255,169 @@ struct CaseView {
     int last;           // largest quad index
     float inv_v, cfl;
     bool barrier, tapered, first_face;
-    bool small_steps;   // cfl < 1/2: a step ends in a corner cell of its start quad
+    bool small_steps;   // a step moves under half a cell: it ends in a corner cell of its start quad
 };
 
-// Waveform table position of a clock: interval i and the position w within it in [0, 1)
+// ---- one step (trench_charging_2d.py:584-650) -------------------------------------------
+//
+// Every form of a step below, with the field in shared or in global memory, is built from the
+// same three functions, whose roundings are fixed: packed and _rn operations and fmaf are never
+// contracted or split by the compiler, so a particle's path does not depend on the form that
+// stepped it, the launch shape or where the field lies.
+
+// Adding MAGIC (2^23 + 2^22 + 1, odd) to a value below 2^22 rounds it to an integer, which the low
+// mantissa bits then hold: to the nearest (one half upwards from an even integer), or, rounded
+// down, to its floor.  One packed add for two floors or conversions, which run at a quarter of
+// its rate.
+constexpr float MAGIC = 12582913.f;
+constexpr int MAGIC_BITS = 0x4b400001;
+__device__ __forceinline__ int magic_int(float r) { return __float_as_int(r) - MAGIC_BITS; }
+__device__ __forceinline__ float2 magic_value(float2 r) { return __fadd2_rn(r, make_float2(-MAGIC, -MAGIC)); }
+__device__ __forceinline__ float2 magic_floor(float2 a) {
+    float2 r;
+    asm("{\n\t.reg .b64 x, m, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 m, {%4, %4};\n\t"
+        "add.rm.ftz.f32x2 z, x, m;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(MAGIC));
+    return r;
+}
+// a - b of packed pairs, exact where b is a's integer part.
+__device__ __forceinline__ float2 minus2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+
+// The quad of a particle, the corners (ix - 1 + hx, iy - 1 + hy) .. + 1 where h says whether the
+// offset is in the cell's upper half (in the halo-padded field this needs no wrap, and the
+// clipped rows one clamp), and its position between them, o + 1/2 - h.
+template <bool SMEM, int RF>
+__device__ __forceinline__ void load_quad(const K32 &k, const CaseView<SMEM> &C, const LaneState &s, QuadCache &q) {
+    int col;
+    if (SMEM) {
+        const float2 r = __fadd2_rn(s.o, make_float2(MAGIC, MAGIC));
+        q.t = __fadd2_rn(minus2(s.o, magic_value(r)), make_float2(0.5f, 0.5f));
+        col = s.ix + magic_int(r.x);
+        q.row = s.iy + magic_int(r.y);
+    } else {
+        // fewer operations in a row, for steps that wait for the loads
+        const bool hx = s.o.x >= 0.5f, hy = s.o.y >= 0.5f;
+        q.t = __fadd2_rn(s.o, make_float2(hx ? -0.5f : 0.5f, hy ? -0.5f : 0.5f));
+        col = s.ix + hx;
+        q.row = s.iy + hy;
+    }
+    q.template load<SMEM, RF>(C.F, k.rf_field, col * C.P + max(q.row, 0), C.P, C.last);
+}
+
+// 1 / (sum of the vacuum corners' weights): solid corners are left out of the field's average.
+__device__ __forceinline__ float vacuum_weight(const QuadCache &q) {
+    const float v00 = vac_of(q.c00), v01 = vac_of(q.c01), v10 = vac_of(q.c10), v11 = vac_of(q.c11);
+    const float s0 = fmaf(q.t.y, v01 - v00, v00), s1 = fmaf(q.t.y, v11 - v10, v10);
+    return __fdividef(1.f, fmaxf(fmaf(q.t.x, s1 - s0, s0), 1e-12f));
+}
+
+// Waveform table position of a clock: interval i and the position within it
 // (trench_rf.py:5-11: periodic linear interpolation of n_phase samples; the last interval
-// runs to the first sample).  The clock is a 32-bit fraction of the period, so clock x
-// n_phase is the table position as a 32.32 fixed-point number: the high word is the
-// interval, the top 23 bits of the low word are the mantissa of 1 + w.
+// runs to the first sample).
 __device__ __forceinline__ int rf_interval(const K32 &k, uint32_t clock, float &w) {
-    const unsigned long long f = (unsigned long long)clock * (unsigned)k.a.n_phase;
-    w = __uint_as_float(0x3f800000u | ((uint32_t)f >> 9)) - 1.f;
-    return (int)(f >> 32);
+    const float c = (float)clock;
+    const int i = min((int)__fmul_rn(c, k.wave_scale), k.a.n_phase - 1);  // a clock just below 2^32 may round up to n
+    w = fmaf(c, k.wave_scale, -(float)i);
+    return i;
 }
 
-// Voltage deltas (substrate, mask) of the waveform at a clock.
-__device__ __forceinline__ void rf_voltages(const K32 &k, uint32_t clock, float &vs, float &vm) {
-    float w;
-    const float4 e = __ldg(k.rf_wave + rf_interval(k, clock, w));
-    vs = fmaf(w, e.z, e.x);
-    vm = fmaf(w, e.w, e.y);
+// Acceleration A, time step and (circuit_rf) clock advance of a particle's next step
+// (trench_charging_2d.py:492-509, 587-608): vacuum-weighted bilinear field, with inv_sw =
+// vacuum_weight (1 in an open quad), and the CFL step dt = cfl / (|v| + sqrt(2 |a|) + 1 m/s).
+template <int RF, bool SMEM>
+__device__ __forceinline__ void step_size(const K32 &k, const CaseView<SMEM> &C, const LaneState &s,
+                                          QuadCache &q, float inv_sw, float2 &A, float &dt, uint32_t &inc) {
+    const float tx = q.t.x, ty = q.t.y;
+    const float2 M1 = make_float2(-1.f, -1.f), txx = make_float2(tx, tx), tyy = make_float2(ty, ty);
+    const float2 f00 = make_float2(q.c00.ex, q.c00.ey), f01 = make_float2(q.c01.ex, q.c01.ey);
+    const float2 f10 = make_float2(q.c10.ex, q.c10.ey), f11 = make_float2(q.c11.ex, q.c11.ey);
+    // bilinear sum of (ex, ey) as one packed pair: along y in both columns, then along x
+    const float2 y0 = __ffma2_rn(tyy, __ffma2_rn(f00, M1, f01), f00);
+    const float2 y1 = __ffma2_rn(tyy, __ffma2_rn(f10, M1, f11), f10);
+    const float2 E = __ffma2_rn(txx, __ffma2_rn(y0, M1, y1), y0);
+    const float speed = sqrtf(fmaf(s.v.x, s.v.x, __fmul_rn(s.v.y, s.v.y)));
+    const float qs = __fmul_rn(s.qm, inv_sw);
+    const float2 qss = make_float2(qs, qs);
+    inc = 0u;
+    if (!RF) {
+        A = __fmul2_rn(qss, E);
+        const float acc = sqrtf(fmaf(A.x, A.x, __fmul_rn(A.y, A.y)));
+        dt = __fdividef(C.cfl, __fadd_rn(__fadd_rn(speed, sqrtf(__fmul_rn(2.f, acc))), C.inv_v));
+    } else {
+        // in-flight RF field (trench_trace.cu:97-110): the basis fields at the same corners
+        // and weights bound the step, and the field is taken at the mid-step clock.  The
+        // waveform interval of the start clock is loaded before the step is known: a
+        // CFL-limited step is far shorter than an interval, so the mid-step clock is
+        // nearly always in it and the lookup leaves the step's dependency chain.
+        const uint32_t c0 = s.clock;
+        float w0;
+        const int i0 = rf_interval(k, c0, w0);
+        const float4 e0 = __ldg(k.rf_wave + i0);
+        if (RF == RF_STEP && SMEM) q.load_basis(k.rf_field, C.P);
+        const float4 b00 = q.b00, b01 = q.b01, b10 = q.b10, b11 = q.b11;
+        const float ux = __fsub_rn(1.f, tx), uy = __fsub_rn(1.f, ty);
+        const float w00 = __fmul_rn(ux, uy), w10 = __fmul_rn(tx, uy), w01 = __fmul_rn(ux, ty), w11 = __fmul_rn(tx, ty);
+        const float2 p00 = make_float2(w00, w00), p10 = make_float2(w10, w10), p01 = make_float2(w01, w01),
+                     p11 = make_float2(w11, w11);
+        // weighted sums like the field's; the vacuum normalisation is applied once
+        float2 Es = __ffma2_rn(p00, make_float2(b00.x, b00.y), __fmul2_rn(p10, make_float2(b10.x, b10.y)));
+        float2 Em = __ffma2_rn(p00, make_float2(b00.z, b00.w), __fmul2_rn(p10, make_float2(b10.z, b10.w)));
+        Es = __ffma2_rn(p11, make_float2(b11.x, b11.y), __ffma2_rn(p01, make_float2(b01.x, b01.y), Es));
+        Em = __ffma2_rn(p11, make_float2(b11.z, b11.w), __ffma2_rn(p01, make_float2(b01.z, b01.w), Em));
+        const float bx = __fadd_rn(fabsf(E.x), fmaf(k.bvs, fabsf(Es.x), __fmul_rn(k.bvm, fabsf(Em.x))));
+        const float by = __fadd_rn(fabsf(E.y), fmaf(k.bvs, fabsf(Es.y), __fmul_rn(k.bvm, fabsf(Em.y))));
+        const float accel = __fmul_rn(__fmul_rn(fabsf(s.qm), inv_sw), sqrtf(fmaf(bx, bx, __fmul_rn(by, by))));
+        dt = fminf(k.dt_max,
+                   __fdividef(C.cfl, __fadd_rn(__fadd_rn(speed, sqrtf(__fmul_rn(2.f, accel))), C.inv_v)));
+        // clock advance in 2^-32 of the period; a step bound below half the period fits 32 bits
+        uint32_t mid;
+        if (k.short_steps) {
+            inc = __float2uint_rn(__fmul_rn(dt, k.t_clock));
+            mid = c0 + (inc >> 1);
+        } else {
+            const unsigned long long w64 = __float2ull_rn(__fmul_rn(dt, k.t_clock));
+            inc = (uint32_t)w64;
+            mid = c0 + (uint32_t)(w64 >> 1);
+        }
+        float w;
+        const int im = rf_interval(k, mid, w);
+        const float4 e = im == i0 ? e0 : __ldg(k.rf_wave + im);
+        const float vs = fmaf(w, e.z, e.x), vm = fmaf(w, e.w, e.y);
+        const float2 sum = __ffma2_rn(make_float2(vs, vs), Es, __fmul2_rn(make_float2(vm, vm), Em));
+        A = __fmul2_rn(qss, __fadd2_rn(E, sum));
+    }
 }
 
-// Bilinear sum of a packed pair over a quad's corners: along y in both columns, then along x.
-__device__ __forceinline__ float2 bilinear2(float2 f00, float2 f01, float2 f10, float2 f11, float2 tx, float2 ty) {
-    const float2 M1 = make_float2(-1.f, -1.f);
-    const float2 e0 = __ffma2_rn(ty, __ffma2_rn(f00, M1, f01), f00);
-    const float2 e1 = __ffma2_rn(ty, __ffma2_rn(f10, M1, f11), f10);
-    return __ffma2_rn(tx, __ffma2_rn(e0, M1, e1), e0);
+// v' = v + a dt, the move S = (v + v') dt / 2 = (v + a dt / 2) dt and the position after it, from
+// the cell's corner: in (-1, 2), a step moves less than a cell.
+struct Move {
+    float2 v, S, pos;
+};
+__device__ __forceinline__ Move move_by(const K32 &k, const LaneState &s, float2 A, float dt) {
+    Move m;
+    const float2 dtt = make_float2(dt, dt);
+    const float hdt = __fmul_rn(0.5f, dt);
+    const float2 mean = __ffma2_rn(A, make_float2(hdt, hdt), s.v);
+    m.v = __ffma2_rn(A, dtt, s.v);
+    // the product alone: packed products are contracted with a sum that follows, whatever their
+    // rounding modifiers, but not a fused one with an addend (-0) that the compiler cannot know
+    m.S = __ffma2_rn(mean, dtt, make_float2(k.minus_zero, k.minus_zero));
+    m.pos = __fadd2_rn(s.o, m.S);
+    return m;
 }
-
-// Column position of a particle in [0, nx) cells.
-__device__ __forceinline__ double wrap_column(double x, int nx) {
-    return x < 0.0 ? x + nx : (x >= nx ? x - nx : x);
+// Offset in the new cell: the remainder, which may round up to 1 and is kept below it (so is that
+// of a position that is not a number).
+__device__ __forceinline__ float2 offset_in(float2 pos, float2 cell) {
+    const float2 rem = minus2(pos, cell);
+    return make_float2(fminf(rem.x, ONE_BELOW), fminf(rem.y, ONE_BELOW));
+}
+// Periodic x: whatever is beyond the grid wraps to its other side; for columns -1 .. nx in two
+// instructions (as unsigned, the wrapped index is the smaller).
+__device__ __forceinline__ int wrap_column(int c, int nx) { return c < 0 ? nx - 1 : (c >= nx ? 0 : c); }
+__device__ __forceinline__ int wrap_next(int c, int nx) {
+    const unsigned a = __viaddmin_u32((unsigned)c, (unsigned)nx, (unsigned)c);
+    return (int)__viaddmin_u32(a, (unsigned)-nx, a);
 }
 
 // Writes the outputs of a particle that is absorbed (1), escaped (2) or stopped at its step
@@ -338,8 +434,8 @@ __device__ __forceinline__ void finish_particle(const K32 &k, LaneState &s, Lane
         a.d_status[pid] = (int8_t)done;
     }
     if (done == 3 || a.write_state) {
-        a.d_x[pid] = wrap_column((double)s.cx + (double)s.u.x, k.nx) * k.dx;
-        a.d_y[pid] = ((double)s.cy + (double)s.u.y) * k.dx;
+        a.d_x[pid] = ((double)s.ix + (double)s.o.x) * k.dx;
+        a.d_y[pid] = ((double)s.iy + (double)s.o.y) * k.dx;
         a.d_vx[pid] = (double)s.v.x * k.vscale;
         a.d_vy[pid] = (double)s.v.y * k.vscale;
     }
@@ -348,182 +444,90 @@ __device__ __forceinline__ void finish_particle(const K32 &k, LaneState &s, Lane
         a.d_clock[2 * pid + 1] = (double)s.elapsed;
     }
     s.pid = -1;
+    s.iy = 0;                       // an empty lane's quad stays in the grid
 }
 
-// Quad of a particle: its vertex, or in the cell frame the vertex nearest to its offset.
+// One step of one particle with everything it may meet: escape, staircase corner, first-face
+// wall entry, barrier reflection, the step cap; an ended particle's outputs are written and
+// s.pid becomes -1.  Fields in global memory take every step here: those steps wait for the
+// field's loads, and one branch a step costs less than lanes that three forms hold back.
 template <bool SMEM, int RF>
-__device__ __forceinline__ void load_quad(const K32 &k, const CaseView<SMEM> &C, const LaneState &s, QuadCache &q) {
-    int at = s.cx * C.P + s.cy;
-    if (!SMEM) at = (s.cx + (s.u.x >= 0.5f ? 1 : 0)) * C.P + max(s.cy + (s.u.y >= 0.5f ? 1 : 0), 0);
-    q.template load<SMEM, RF>(C.F, k.rf_field, at, C.P, C.last);
-}
-
-// ---- the cell frame: fields in global memory ---------------------------------------------
-
-// Waveform table position of a clock: interval i and the position within it.
-__device__ __forceinline__ int cell_rf_interval(const K32 &k, uint32_t clock, float &w) {
-    const float f = (float)clock * k.wave_scale;
-    const int i = min((int)f, k.a.n_phase - 1);  // a clock just below 2^32 may round up to n
-    w = f - (float)i;
-    return i;
-}
-
-// Acceleration A, time step and clock advance of the next step (see step_size).
-template <int RF>
-__device__ __forceinline__ void cell_step_size(const K32 &k, const CaseView<false> &C, const LaneState &s,
-                                               const QuadCache &q, bool near, float2 &A, float &dt, uint32_t &inc) {
-    const float2 tq = __fadd2_rn(s.u, make_float2(s.u.x >= 0.5f ? -0.5f : 0.5f, s.u.y >= 0.5f ? -0.5f : 0.5f));
-    const float tx = tq.x, ty = tq.y;
-    const tb_fcell c00 = q.c00, c01 = q.c01, c10 = q.c10, c11 = q.c11;
-    const float2 E = bilinear2(make_float2(c00.ex, c00.ey), make_float2(c01.ex, c01.ey), make_float2(c10.ex, c10.ey),
-                               make_float2(c11.ex, c11.ey), make_float2(tx, tx), make_float2(ty, ty));
-    float inv_sw = 1.f;
-    if (near) {
-        const float v00 = vac_of(c00), v01 = vac_of(c01), v10 = vac_of(c10), v11 = vac_of(c11);
-        const float s0 = fmaf(ty, v01 - v00, v00), s1 = fmaf(ty, v11 - v10, v10);
-        inv_sw = __fdividef(1.f, fmaxf(fmaf(tx, s1 - s0, s0), 1e-12f));
-    }
-    const float speed = sqrtf(fmaf(s.v.x, s.v.x, s.v.y * s.v.y));
-    const float qs = s.hq * inv_sw;
-    inc = 0u;
-    if (!RF) {
-        A = __fmul2_rn(make_float2(qs, qs), E);
-        const float acc = sqrtf(fmaf(A.x, A.x, A.y * A.y));
-        dt = __fdividef(C.cfl, speed + sqrtf(2.f * acc) + C.inv_v);
-    } else {
-        // in-flight RF field (trench_trace.cu:97-110), as step_size
-        const int base = q.base, P = C.P;
-        const float ux = 1.f - tx, uy = 1.f - ty;
-        const float w00 = ux * uy, w10 = tx * uy, w01 = ux * ty, w11 = tx * ty;
-        const uint32_t c0 = s.clock;
-        float w0;
-        const int i0 = cell_rf_interval(k, c0, w0);
-        const float4 e0 = __ldg(k.rf_wave + i0);
-        const float4 b00 = __ldg(k.rf_field + base), b01 = __ldg(k.rf_field + base + 1);
-        const float4 b10 = __ldg(k.rf_field + base + P), b11 = __ldg(k.rf_field + base + P + 1);
-        const float sxs = w00 * b00.x + w10 * b10.x + w01 * b01.x + w11 * b11.x;
-        const float sys = w00 * b00.y + w10 * b10.y + w01 * b01.y + w11 * b11.y;
-        const float sxm = w00 * b00.z + w10 * b10.z + w01 * b01.z + w11 * b11.z;
-        const float sym = w00 * b00.w + w10 * b10.w + w01 * b01.w + w11 * b11.w;
-        const float bx = fabsf(E.x) + (k.bvs * fabsf(sxs) + k.bvm * fabsf(sxm));
-        const float by = fabsf(E.y) + (k.bvs * fabsf(sys) + k.bvm * fabsf(sym));
-        const float accel = fabsf(s.hq) * inv_sw * sqrtf(bx * bx + by * by);
-        dt = fminf(k.dt_max, __fdividef(C.cfl, speed + sqrtf(2.f * accel) + C.inv_v));
-        uint32_t mid;
-        if (k.short_steps) {
-            inc = __float2uint_rn(dt * k.t_clock);
-            mid = c0 + (inc >> 1);
-        } else {
-            const unsigned long long w64 = __float2ull_rn(dt * k.t_clock);
-            inc = (uint32_t)w64;
-            mid = c0 + (uint32_t)(w64 >> 1);
-        }
-        float w;
-        const int im = cell_rf_interval(k, mid, w);
-        const float4 e = im == i0 ? e0 : __ldg(k.rf_wave + im);
-        const float vs = fmaf(w, e.z, e.x), vm = fmaf(w, e.w, e.y);
-        A = make_float2(qs * (E.x + (vs * sxs + vm * sxm)), qs * (E.y + (vs * sys + vm * sym)));
-    }
-}
-
-// v' = v + a dt and the move (v + v') dt / 2 = (v + a dt / 2) dt.  A step moves less than one cell, so
-// the new offset lies in (-1, 2): the cell change is its floor and the new offset the
-// remainder (a remainder that rounds up to 1 is clamped below 1).  Compares in place of the
-// floors and conversions: 3150 -> 3280 us a batch (200 x 700 cells, 2^19 particles).
-struct CellMove {
-    float2 v, S, o;
-    int dix, nix, niy;
-};
-// a + b, never contracted with the product that made b (an add with a rounding modifier is not).
-__device__ __forceinline__ float2 add2_alone(float2 a, float2 b) {
-    float2 r;
-    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
-        "add.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
-        : "=f"(r.x), "=f"(r.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return r;
-}
-__device__ __forceinline__ CellMove cell_move(const CaseView<false> &C, const LaneState &s, float2 A, float dt) {
-    CellMove m;
-    const float2 dtt = make_float2(dt, dt);
-    const float hdt = 0.5f * dt;
-    m.v = __ffma2_rn(A, dtt, s.v);
-    m.S = __fmul2_rn(__ffma2_rn(A, make_float2(hdt, hdt), s.v), dtt);
-    const float2 pos = add2_alone(s.u, m.S);
-    const float fnx = floorf(pos.x), fny = floorf(pos.y);
-    const float2 rem = __ffma2_rn(make_float2(fnx, fny), make_float2(-1.f, -1.f), pos);
-    m.o = make_float2(fminf(rem.x, ONE_BELOW), fminf(rem.y, ONE_BELOW));
-    m.dix = (int)fnx;
-    const int nix = s.cx + m.dix;
-    m.nix = nix < 0 ? C.nx - 1 : (nix >= C.nx ? 0 : nix);
-    m.niy = s.cy + (int)fny;
-    return m;
-}
-
-// One step of one particle (trench_charging_2d.py:584-650), as step_open and step_decide
-// together; these steps wait for the field's loads, and one branch a step costs less than the
-// lanes that three forms hold back.
-template <int RF>
-__device__ __forceinline__ void cell_step(const K32 &k, const CaseView<false> &C, LaneState &s, LaneTally &t,
+__device__ __forceinline__ void step_full(const K32 &k, const CaseView<SMEM> &C, LaneState &s, LaneTally &t,
                                           QuadCache &q) {
     const tb_trace_args &a = k.a;
-    const int ny = C.ny, P = C.P;
-    load_quad<false, RF>(k, C, s, q);
+    const int nx = C.nx, ny = C.ny, P = C.P;
+    load_quad<SMEM, RF>(k, C, s, q);
     // a step below half a cell ends in a corner cell of its quad
     const bool near = !(C.small_steps && is_open(q.c00));
     float2 A;
     float dt;
     uint32_t inc;
-    cell_step_size<RF>(k, C, s, q, near, A, dt, inc);
-    const CellMove m = cell_move(C, s, A, dt);
+    // circuit_rf: the basis fields' loads go out before a branch waits for the field's, and there
+    // is no branch for the weight (3000 + 3000 particles on 120 x 560 cells: 5050 -> 4205 us a
+    // batch); without RF the branch is the better one (200 x 700 cells: 3165 us, 3325 without it)
+    float weight = 1.f;
+    if (RF) {
+        if (RF == RF_STEP && !SMEM) q.load_basis(k.rf_field, P);
+        const float w = vacuum_weight(q);
+        weight = near ? w : 1.f;
+    } else if (near) {
+        weight = vacuum_weight(q);
+    }
+    step_size<RF>(k, C, s, q, weight, A, dt, inc);
+    const Move m = move_by(k, s, A, dt);
+    // the cell change; a move that is not a number changes neither column nor row
+    const float fnx = floorf(m.pos.x), fny = floorf(m.pos.y);
+    const int dix = (int)fnx, niy = s.iy + (int)fny;
+    const int nix = wrap_column(s.ix + dix, nx);
+    const float2 no = offset_in(m.pos, make_float2(fnx, fny));
     if (RF) {
         s.clock += inc;
-        s.elapsed += dt * k.t_sec;
+        s.elapsed = fmaf(dt, k.t_sec, s.elapsed);
     }
     ++s.steps;
-    const bool escaped = m.niy >= ny;
+    const bool escaped = niy >= ny;
     bool hit = false, corner = false;
     if (near && !escaped) {
-        if (C.small_steps && s.cy >= 0) {
-            // the end cell is a corner of the quad
-            const bool right = m.dix >= (s.u.x >= 0.5f ? 1 : 0), above = m.niy - s.cy >= (s.u.y >= 0.5f ? 1 : 0);
+        if (!SMEM && C.small_steps && s.iy >= 0) {
+            // the end cell is a corner of the quad (saves a load from global memory)
+            const bool right = dix >= (s.o.x >= 0.5f ? 1 : 0), above = niy - s.iy >= (s.o.y >= 0.5f ? 1 : 0);
             const float f = right ? (above ? q.c11.ex : q.c10.ex) : (above ? q.c01.ex : q.c00.ex);
             hit = !(__float_as_uint(f) & 1u);
         } else {
-            hit = !C.F.vac((m.nix + 1) * P + max(m.niy, -1) + 1);
+            hit = !C.F.vac((nix + 1) * P + max(niy, -1) + 1);
         }
         // both the column and the (clipped) row changed: a staircase corner may lie on the path
         // between two vacuum cells (trench_charging_2d.py:614-621).  The move reaches the wall
         // only if the cell beyond the first boundary crossed is solid (the first-face rule
         // below, same expressions).
-        corner = C.tapered && !hit && m.dix != 0 && max(m.niy, 0) != max(s.cy, 0);
+        corner = C.tapered && !hit && dix != 0 && max(niy, 0) != max(s.iy, 0);
         if (corner) {
-            const int y0c = min(max(s.cy, 0), ny - 1), iyn = min(max(m.niy, 0), ny - 1);
-            const float fx = ((m.dix > 0 ? 1.f : 0.f) - s.u.x) / m.S.x;
-            const float fy = ((iyn > y0c ? 1.f : 0.f) - s.u.y) / m.S.y;
+            const int y0c = min(max(s.iy, 0), ny - 1), iyn = min(max(niy, 0), ny - 1);
+            const float fx = __fsub_rn(dix > 0 ? 1.f : 0.f, s.o.x) / m.S.x;
+            const float fy = __fsub_rn(iyn > y0c ? 1.f : 0.f, s.o.y) / m.S.y;
             const bool x_first = fx < fy;
-            corner = !C.F.vac((x_first ? m.nix + 1 : s.cx + 1) * P + (x_first ? y0c : iyn) + 1);
+            corner = !C.F.vac((x_first ? nix + 1 : s.ix + 1) * P + (x_first ? y0c : iyn) + 1);
         }
     }
     if (!(hit || corner || escaped || s.steps >= s.stop_at)) {
-        s.cx = m.nix; s.cy = m.niy; s.u = m.o; s.v = m.v;
+        s.ix = nix; s.iy = niy; s.o = no; s.v = m.v;
         return;
     }
 
     // wall contact, escape or step cap
-    const int y0c = min(max(s.cy, 0), ny - 1), iyn = min(max(m.niy, 0), ny - 1);
+    const int y0c = min(max(s.iy, 0), ny - 1), iyn = min(max(niy, 0), ny - 1);
     const int diy = iyn - y0c;       // rows clipped like the reference
-    int dcell = m.nix * ny + iyn;
+    int dcell = nix * ny + iyn;
     bool reflected = false;
     if (hit ? C.first_face : corner) {
         // first solid face crossed (trench_charging_2d.py:512-539) in cell units
         const float inf = __int_as_float(0x7f800000);
-        const float fx = m.dix != 0 ? ((m.dix > 0 ? 1.f : 0.f) - s.u.x) / m.S.x : inf;
-        const float fy = diy != 0 ? ((diy > 0 ? 1.f : 0.f) - s.u.y) / m.S.y : inf;
+        const float fx = dix != 0 ? __fsub_rn(dix > 0 ? 1.f : 0.f, s.o.x) / m.S.x : inf;
+        const float fy = diy != 0 ? __fsub_rn(diy > 0 ? 1.f : 0.f, s.o.y) / m.S.y : inf;
         const bool x_first = fx < fy;
-        const int ax_ = x_first ? m.nix : s.cx, ay_ = x_first ? y0c : y0c + diy;
-        const bool use_last = m.dix != 0 && diy != 0 && C.F.vac((ax_ + 1) * P + ay_ + 1);
-        const int cx = use_last ? m.nix : ax_, cy = use_last ? y0c + diy : ay_;
+        const int ax_ = x_first ? nix : s.ix, ay_ = x_first ? y0c : y0c + diy;
+        const bool use_last = dix != 0 && diy != 0 && C.F.vac((ax_ + 1) * P + ay_ + 1);
+        const int cx = use_last ? nix : ax_, cy = use_last ? y0c + diy : ay_;
         const bool face_x = use_last ? !x_first : x_first;
         const int ccell = cx * ny + cy;
         hit = !C.F.vac((cx + 1) * P + cy + 1);
@@ -531,20 +535,20 @@ __device__ __forceinline__ void cell_step(const K32 &k, const CaseView<false> &C
         if (hit && C.barrier) {
             const float4 b = __ldg(k.barrier + ccell);
             // neighbour the particle came from: W/E across an x face, S/N across a y face
-            float dphi = face_x ? (m.dix > 0 ? b.x : b.y) : (diy > 0 ? b.z : b.w);
+            float dphi = face_x ? (dix > 0 ? b.x : b.y) : (diy > 0 ? b.z : b.w);
             if (RF) {
                 // barrier of the instantaneous potential at the clock after the step
                 // (trench_trace.cu:131-136)
                 float w;
-                const float4 e = __ldg(k.rf_wave + cell_rf_interval(k, s.clock, w));
+                const float4 e = __ldg(k.rf_wave + rf_interval(k, s.clock, w));
                 const float vs = fmaf(w, e.z, e.x), vm = fmaf(w, e.w, e.y);
                 const float4 bs = __ldg(k.rf_barrier + ccell), bm = __ldg(k.rf_barrier + C.cells + ccell);
-                const float ds = face_x ? (m.dix > 0 ? bs.x : bs.y) : (diy > 0 ? bs.z : bs.w);
-                const float dm = face_x ? (m.dix > 0 ? bm.x : bm.y) : (diy > 0 ? bm.z : bm.w);
-                dphi += vs * ds + vm * dm;
+                const float ds = face_x ? (dix > 0 ? bs.x : bs.y) : (diy > 0 ? bs.z : bs.w);
+                const float dm = face_x ? (dix > 0 ? bm.x : bm.y) : (diy > 0 ? bm.z : bm.w);
+                dphi = __fadd_rn(dphi, fmaf(vs, ds, __fmul_rn(vm, dm)));
             }
             const float vn = face_x ? m.v.x : m.v.y;
-            if (0.5f * vn * vn < s.hq * dphi) {
+            if (0.5f * vn * vn < s.qm * dphi) {
                 // reflect: the normal velocity flips, the position stays at the start point
                 s.v.x = face_x ? -m.v.x : m.v.x;
                 s.v.y = face_x ? m.v.y : -m.v.y;
@@ -553,293 +557,8 @@ __device__ __forceinline__ void cell_step(const K32 &k, const CaseView<false> &C
             }
         }
     }
-    if (!reflected) { s.cx = m.nix; s.cy = m.niy; s.u = m.o; s.v = m.v; }
-    int done = 0;
+    if (!reflected) { s.ix = nix; s.iy = niy; s.o = no; s.v = m.v; }
     if (hit) {
-        if (dcell < 0 || dcell >= C.cells) {
-            atomicCAS(k.err, TB_DERR_NONE, TB_DERR_BAD_CELL);
-        } else {
-            tb_deposit(a.d_counts, (size_t)s.spc * C.cells + dcell);
-        }
-        if (a.d_hit) a.d_hit[s.pid] = dcell;
-        if (s.spc == 0) ++t.hit_i; else ++t.hit_e;
-        done = 1;
-    } else if (escaped && !reflected) {
-        if (s.spc == 0) ++t.esc_i; else ++t.esc_e;
-        done = 2;
-    } else if (s.steps >= s.stop_at) {
-        done = 3;
-    }
-    if (done) finish_particle<RF>(k, s, t, done);
-}
-
-// ---- the vertex frame: fields in shared memory -------------------------------------------
-
-// Half acceleration h, time step and (circuit_rf) clock advance of a particle's next step
-// (trench_charging_2d.py:492-509, 587-608): vacuum-weighted bilinear field and the CFL step
-// dt = cfl / (|v| + sqrt(2 |a|) + 1 m/s), with sqrt(2 |a|) = 2 (|h|^2)^(1/4).  NEAR: the quad may
-// hold solid corners, whose weights are left out; otherwise the vacuum weights sum to one.
-template <int RF, bool NEAR>
-__device__ __forceinline__ void step_size(const K32 &k, const CaseView<true> &C, const LaneState &s,
-                                          const QuadCache &q, float2 &h, float &dt, uint32_t &inc) {
-    const float tx = s.u.x + 0.5f, ty = s.u.y + 0.5f;
-    const float2 txx = make_float2(tx, tx), tyy = make_float2(ty, ty);
-    const tb_fcell c00 = q.c00, c01 = q.c01, c10 = q.c10, c11 = q.c11;
-    float2 E = bilinear2(make_float2(c00.ex, c00.ey), make_float2(c01.ex, c01.ey), make_float2(c10.ex, c10.ey),
-                         make_float2(c11.ex, c11.ey), txx, tyy);
-    float hqs = s.hq;
-    if (NEAR) {
-        // no branch: some lane of the warp needs it, and an open quad's own value is selected
-        const float v00 = vac_of(c00), v01 = vac_of(c01), v10 = vac_of(c10), v11 = vac_of(c11);
-        const float s0 = fmaf(ty, v01 - v00, v00), s1 = fmaf(ty, v11 - v10, v10);
-        const float hqn = __fdividef(hqs, fmaxf(fmaf(tx, s1 - s0, s0), 1e-12f));
-        hqs = is_open(c00) ? hqs : hqn;
-    }
-    const float speed = sqrtf(fmaf(s.v.x, s.v.x, s.v.y * s.v.y)) + C.inv_v;
-    inc = 0u;
-    if (!RF) {
-        h = __fmul2_rn(make_float2(hqs, hqs), E);
-        dt = __fdividef(C.cfl, fmaf(2.f, sqrtf(sqrtf(fmaf(h.x, h.x, h.y * h.y))), speed));
-    } else {
-        // in-flight RF field (trench_trace.cu:97-110): the basis fields at the same corners
-        // and weights bound the step, and the field is taken at the mid-step clock.  The
-        // waveform interval of the start clock is loaded before the step is known: a
-        // CFL-limited step is far shorter than an interval, so the mid-step clock is
-        // nearly always in it and the lookup leaves the step's dependency chain.
-        const uint32_t c0 = s.clock;
-        const int base = q.base, P = C.P;
-        float w0;
-        const int i0 = rf_interval(k, c0, w0);
-        const float4 e0 = __ldg(k.rf_wave + i0);
-        float4 b00 = q.b00, b01 = q.b01, b10 = q.b10, b11 = q.b11;
-        if (RF == RF_STEP) {
-            b00 = __ldg(k.rf_field + base); b01 = __ldg(k.rf_field + base + 1);
-            b10 = __ldg(k.rf_field + base + P); b11 = __ldg(k.rf_field + base + P + 1);
-        }
-        const float2 Es = bilinear2(make_float2(b00.x, b00.y), make_float2(b01.x, b01.y), make_float2(b10.x, b10.y),
-                                    make_float2(b11.x, b11.y), txx, tyy);
-        const float2 Em = bilinear2(make_float2(b00.z, b00.w), make_float2(b01.z, b01.w), make_float2(b10.z, b10.w),
-                                    make_float2(b11.z, b11.w), txx, tyy);
-        const float bx = hqs * (fabsf(E.x) + fmaf(k.bvs, fabsf(Es.x), k.bvm * fabsf(Em.x)));
-        const float by = hqs * (fabsf(E.y) + fmaf(k.bvs, fabsf(Es.y), k.bvm * fabsf(Em.y)));
-        dt = fminf(k.dt_max, __fdividef(C.cfl, fmaf(2.f, sqrtf(sqrtf(fmaf(bx, bx, by * by))), speed)));
-        // clock advance in 2^-32 of the period; a step bound below the period fits 32 bits
-        uint32_t mid;
-        if (k.short_steps) {
-            inc = __float2uint_rn(dt * k.t_clock);
-            mid = c0 + (inc >> 1);
-        } else {
-            const unsigned long long w64 = __float2ull_rn(dt * k.t_clock);
-            inc = (uint32_t)w64;
-            mid = c0 + (uint32_t)(w64 >> 1);
-        }
-        float w;
-        const int im = rf_interval(k, mid, w);
-        const float4 e = im == i0 ? e0 : __ldg(k.rf_wave + im);
-        const float vs = fmaf(w, e.z, e.x), vm = fmaf(w, e.w, e.y);
-        E = __ffma2_rn(make_float2(vs, vs), Es, E);
-        E = __ffma2_rn(make_float2(vm, vm), Em, E);
-        h = __fmul2_rn(make_float2(hqs, hqs), E);
-    }
-}
-
-// New offset from the present vertex, x + v dt + h dt^2, in (-1.5, 1.5).
-__device__ __forceinline__ float2 moved(const LaneState &s, float2 h, float dt) {
-    const float dd = dt * dt;
-    return __ffma2_rn(h, make_float2(dd, dd), __ffma2_rn(s.v, make_float2(dt, dt), s.u));
-}
-// Its nearest integers (the vertex change) as rounded sums, see MAGIC, and the remainders (exact).
-__device__ __forceinline__ float2 rounded(float2 p) { return __fadd2_rn(p, make_float2(MAGIC, MAGIC)); }
-__device__ __forceinline__ float2 remainder2(float2 p, float2 r) {
-    return __ffma2_rn(__fadd2_rn(r, make_float2(-MAGIC, -MAGIC)), make_float2(-1.f, -1.f), p);
-}
-__device__ __forceinline__ int vertex_change(float r) { return __float_as_int(r) - MAGIC_BITS; }
-// periodic x: vertices -1 and nx + 1 wrap (as unsigned, the wrapped index is the smaller)
-__device__ __forceinline__ int wrap_vertex(int c, int nx) {
-    const unsigned a = __viaddmin_u32((unsigned)c, (unsigned)nx, (unsigned)c);
-    return (int)__viaddmin_u32(a, (unsigned)-nx, a);
-}
-
-// Takes a step of length dt to offset p (r = rounded(p)) from the present vertex.
-template <int RF>
-__device__ __forceinline__ void take_step(const K32 &k, const CaseView<true> &C, LaneState &s, QuadCache &q, float2 h,
-                                          float dt, uint32_t inc, float2 p, float2 r) {
-    const float d2 = dt + dt;
-    s.cx = wrap_vertex(s.cx + vertex_change(r.x), C.nx);
-    s.cy += vertex_change(r.y);
-    s.v = __ffma2_rn(h, make_float2(d2, d2), s.v);
-    s.u = remainder2(p, r);
-    if (RF) {
-        s.clock += inc;
-        s.elapsed += dt * k.t_sec;
-    }
-    load_quad<true, RF>(k, C, s, q);
-}
-
-// A step of a warp whose lanes' quads are all open: a step moves at most cfl cells (|v| dt +
-// |a| dt^2 / 2 <= cfl for the CFL dt), so with cfl below one half it ends in one of the quad's
-// four corner cells, all vacuum.  Inactive lanes take a step of length zero, which leaves them
-// exactly as they are.
-template <int RF>
-__device__ __forceinline__ void step_open(const K32 &k, const CaseView<true> &C, LaneState &s, QuadCache &q,
-                                          bool active) {
-    float2 h;
-    float dt;
-    uint32_t inc;
-    step_size<RF, false>(k, C, s, q, h, dt, inc);
-    if (!active) {
-        dt = 0.f;
-        inc = 0u;
-    }
-    const float2 p = moved(s, h, dt);
-    take_step<RF>(k, C, s, q, h, dt, inc, p, rounded(p));
-}
-
-// A step of a warp with lanes near a wall or an edge of the grid.  It is taken if it ends in a
-// vacuum cell of the grid with no staircase corner on the way; otherwise the particle stays as
-// it was and the return is false: the step needs the decisions of step_decide.
-template <int RF>
-__device__ __forceinline__ bool step_near(const K32 &k, const CaseView<true> &C, LaneState &s, QuadCache &q,
-                                          bool active) {
-    float2 h;
-    float dt;
-    uint32_t inc;
-    step_size<RF, true>(k, C, s, q, h, dt, inc);
-    float2 p = moved(s, h, dt), r = rounded(p);
-    bool go;
-    if (C.small_steps) {
-        // the end cell is the corner of the quad on the side of the offset's signs
-        const int px = __float_as_int(p.x), py = __float_as_int(p.y);
-        const float f = px < 0 ? (py < 0 ? q.c00.ex : q.c01.ex) : (py < 0 ? q.c10.ex : q.c11.ex);
-        const bool diagonal = C.tapered && ((px ^ __float_as_int(s.u.x)) & (py ^ __float_as_int(s.u.y))) < 0;
-        go = is_open(q.c00) ||
-             ((__float_as_uint(f) & 1u) && (unsigned)(s.cy + (py >> 31)) < (unsigned)C.ny && !diagonal);
-    } else {
-        const float2 un = remainder2(p, r);
-        // padded cell of the end and of the start (a move that is not finite ends nowhere)
-        const int cxw = wrap_vertex(s.cx + vertex_change(r.x), C.nx), cyn = s.cy + vertex_change(r.y);
-        const int ec = cxw + 1 + (__float_as_int(un.x) >> 31), er = cyn + 1 + (__float_as_int(un.y) >> 31);
-        const int sc = s.cx + 1 + (__float_as_int(s.u.x) >> 31), sr = s.cy + 1 + (__float_as_int(s.u.y) >> 31);
-        go = (unsigned)cxw <= (unsigned)C.nx && (unsigned)(er - 1) < (unsigned)C.ny && cyn >= 0 &&
-             C.F.vac(ec * C.P + er) && !(C.tapered && ec != sc && er != sr);
-    }
-    go = go && active;
-    if (!go) {
-        dt = 0.f;
-        inc = 0u;
-        p = s.u;
-        r = make_float2(MAGIC, MAGIC);
-    }
-    take_step<RF>(k, C, s, q, h, dt, inc, p, r);
-    return go;
-}
-
-// One step of one particle with everything it may meet (trench_charging_2d.py:584-650):
-// escape, staircase corner, first-face wall entry, barrier reflection, the step cap (s.steps
-// counts the step already); an ended particle's outputs are written and s.pid becomes -1.
-template <int RF>
-__device__ __forceinline__ void step_decide(const K32 &k, const CaseView<true> &C, LaneState &s, LaneTally &t,
-                                            QuadCache &q) {
-    const int nx = C.nx, ny = C.ny, P = C.P;
-    float2 h;
-    float dt;
-    uint32_t inc;
-    step_size<RF, true>(k, C, s, q, h, dt, inc);
-    const bool near = !(C.small_steps && is_open(q.c00));
-    const float2 p = moved(s, h, dt), r = rounded(p);
-    const float dd = dt * dt, d2 = dt + dt;
-    const float2 vn = __ffma2_rn(h, make_float2(d2, d2), s.v);
-    float2 un = remainder2(p, r);
-    const int cxn = s.cx + vertex_change(r.x);
-    int cyn = s.cy + vertex_change(r.y);
-    int cxw = wrap_vertex(cxn, nx);
-    const tb_trace_args &a = k.a;
-    const float2 move = __ffma2_rn(h, make_float2(dd, dd), __fmul2_rn(s.v, make_float2(dt, dt)));
-    int dix = cxn - s.cx;
-    if (!(fabsf(p.x) < 2.f && fabsf(p.y) < 4e6f)) {
-        // not a finite move: the particle stays where it is until its step cap
-        cxw = s.cx; cyn = s.cy; un = s.u;
-        dix = 0;
-    }
-    cxw = min(max(cxw, 0), nx);   // a one-column grid can step past the wrap
-    if (cyn < 0) {
-        un.y += (float)cyn;
-        cyn = 0;
-    }
-    // padded cell (column, row) of the start and of the end, rows clipped like the
-    // reference; the column and row changes between them
-    const int sx = s.u.x >= 0.f ? 1 : 0, ex = un.x >= 0.f ? 1 : 0;
-    const int sr = min(max(s.cy + (s.u.y >= 0.f ? 1 : 0), 1), ny);
-    const int sc = s.cx + sx, ec = cxw + ex;
-    const int er0 = cyn + (un.y >= 0.f ? 1 : 0);
-    const bool escaped = er0 > ny;
-    const int er = min(max(er0, 1), ny);
-    dix += ex - sx;
-    const int diy = er - sr;
-    bool hit = false, corner = false, x_first = false, reflected = false;
-    if (near && !escaped) {
-        hit = !C.F.vac(ec * P + er);
-        // both the column and the row changed: a staircase corner may lie on the path
-        // between two vacuum cells (trench_charging_2d.py:614-621)
-        corner = C.tapered && !hit && dix != 0 && diy != 0;
-    }
-    int hc = ec, hr = er;            // padded cell of the deposit
-    if (hit ? C.first_face : corner) {
-        // first solid face crossed (trench_charging_2d.py:512-539) in cell units
-        const float inf = __int_as_float(0x7f800000);
-        const float fx = dix != 0 ? ((float)(sx - 1 + (dix > 0 ? 1 : 0)) - s.u.x) / move.x : inf;
-        const float fy = diy != 0 ? ((float)(sr - 1 - s.cy + (diy > 0 ? 1 : 0)) - s.u.y) / move.y : inf;
-        x_first = fx < fy;
-        const int ac = x_first ? ec : sc, ar = x_first ? sr : er;
-        const bool use_last = dix != 0 && diy != 0 && C.F.vac(ac * P + ar);
-        hc = use_last ? ec : ac;
-        hr = use_last ? er : ar;
-        const bool face_x = use_last ? !x_first : x_first;
-        hit = !C.F.vac(hc * P + hr);
-        if (hit && C.barrier) {
-            const int ccell = (hc == 0 ? nx - 1 : hc > nx ? 0 : hc - 1) * ny + hr - 1;
-            const float4 b = __ldg(k.barrier + ccell);
-            // neighbour the particle came from: W/E across an x face, S/N across a y face
-            float dphi = face_x ? (dix > 0 ? b.x : b.y) : (diy > 0 ? b.z : b.w);
-            if (RF) {
-                // barrier of the instantaneous potential at the clock after the step
-                // (trench_trace.cu:131-136)
-                float vs, vm;
-                rf_voltages(k, s.clock + inc, vs, vm);
-                const float4 bs = __ldg(k.rf_barrier + ccell), bm = __ldg(k.rf_barrier + C.cells + ccell);
-                const float ds = face_x ? (dix > 0 ? bs.x : bs.y) : (diy > 0 ? bs.z : bs.w);
-                const float dm = face_x ? (dix > 0 ? bm.x : bm.y) : (diy > 0 ? bm.z : bm.w);
-                dphi += vs * ds + vm * dm;
-            }
-            const float vnorm = face_x ? vn.x : vn.y;
-            if (0.25f * vnorm * vnorm < s.hq * dphi) {
-                // reflect: the normal velocity flips, the position stays at the start point
-                s.v.x = face_x ? -vn.x : vn.x;
-                s.v.y = face_x ? vn.y : -vn.y;
-                if (RF) {
-                    s.clock += inc;
-                    s.elapsed += dt * k.t_sec;
-                }
-                hit = false;
-                reflected = true;
-            }
-        }
-    }
-    if (!reflected) {
-        if (escaped) {              // the quad index stays in the grid
-            un.y += (float)(cyn - ny);
-            cyn = ny;
-        }
-        s.cx = cxw; s.cy = cyn; s.u = un; s.v = vn;
-        if (RF) {
-            s.clock += inc;
-            s.elapsed += dt * k.t_sec;
-        }
-        load_quad<true, RF>(k, C, s, q);
-    }
-
-    if (hit) {
-        const int dcell = (hc == 0 ? nx - 1 : hc > nx ? 0 : hc - 1) * ny + hr - 1;
         if (dcell < 0 || dcell >= C.cells) {
             atomicCAS(k.err, TB_DERR_NONE, TB_DERR_BAD_CELL);
         } else {
@@ -856,9 +575,94 @@ __device__ __forceinline__ void step_decide(const K32 &k, const CaseView<true> &
     }
 }
 
+// ---- fields in shared memory: the two branch-free forms ----------------------------------
+
+// A step of a warp whose active lanes are all in open quads below the top edge: with small steps
+// it ends in one of the quad's four corner cells, all vacuum and in the grid or below it.  Inactive
+// lanes take a step of length zero, which leaves them exactly as they are.
+template <int RF>
+__device__ __forceinline__ void step_open(const K32 &k, const CaseView<true> &C, LaneState &s, QuadCache &q,
+                                          bool active) {
+    float2 A;
+    float dt;
+    uint32_t inc;
+    step_size<RF>(k, C, s, q, 1.f, A, dt, inc);
+    if (!active) {
+        dt = 0.f;
+        inc = 0u;
+    }
+    const Move m = move_by(k, s, A, dt);
+    const float2 r = magic_floor(m.pos), cell = magic_value(r);
+    if (RF) {
+        // (see QuadCache::load: the conversions and the full wrap keep any move's column in the grid)
+        s.ix = wrap_column(s.ix + (int)cell.x, C.nx);
+        s.iy += (int)cell.y;
+    } else if (m.pos.x == m.pos.x && m.pos.y == m.pos.y) {
+        s.ix = wrap_next(s.ix + magic_int(r.x), C.nx);
+        s.iy += magic_int(r.y);
+    }
+    s.v = m.v;
+    s.o = offset_in(m.pos, cell);
+    if (RF) {
+        s.clock += inc;
+        s.elapsed = fmaf(dt, k.t_sec, s.elapsed);
+    }
+    load_quad<true, RF>(k, C, s, q);
+}
+
+// A step of a warp with lanes near a wall or the top edge.  It is taken if it ends in a vacuum
+// cell below the top with no staircase corner on the way; otherwise the particle stays as it was
+// and the return is false: step_full takes that step.
+template <int RF>
+__device__ __forceinline__ bool step_near(const K32 &k, const CaseView<true> &C, LaneState &s, QuadCache &q,
+                                          bool active) {
+    // no branch: some lane of the warp needs the weight, and an open quad's 1 is selected
+    const bool safe = C.small_steps && is_open(q.c00);
+    const float weight = vacuum_weight(q);
+    float2 A;
+    float dt;
+    uint32_t inc;
+    step_size<RF>(k, C, s, q, safe ? 1.f : weight, A, dt, inc);
+    Move m = move_by(k, s, A, dt);
+    bool go;
+    if (C.small_steps) {
+        // the end cell is a corner of the quad (below the grid both rows are copies of row 0)
+        const bool hx = s.o.x >= 0.5f, hy = s.o.y >= 0.5f;
+        const bool right = m.pos.x >= (hx ? 1.f : 0.f), above = m.pos.y >= (hy ? 1.f : 0.f);
+        const float f = right ? (above ? q.c11.ex : q.c10.ex) : (above ? q.c01.ex : q.c00.ex);
+        const bool diagonal = C.tapered && right == hx && above == hy;   // column and row change
+        go = fabsf(m.S.x) < 0.5f && fabsf(m.S.y) < 0.5f && !(above && q.row >= C.ny) &&
+             (safe || ((__float_as_uint(f) & 1u) && !diagonal));
+    } else {
+        const int dix = (int)floorf(m.pos.x), diy = (int)floorf(m.pos.y);
+        const int nix = wrap_column(s.ix + dix, C.nx), niy = s.iy + diy;
+        go = fabsf(m.S.x) < 1.5f && fabsf(m.S.y) < 1.5f && dix >= -1 && dix <= 1 && niy < C.ny &&
+             !(C.tapered && dix != 0 && diy != 0) &&
+             C.F.vac((nix + 1) * C.P + min(max(niy, -1), C.ny) + 1);
+    }
+    go = go && active;
+    if (!go) {
+        m.v = s.v;
+        m.pos = s.o;
+        dt = 0.f;
+        inc = 0u;
+    }
+    const float2 r = magic_floor(m.pos);
+    s.ix = wrap_next(s.ix + magic_int(r.x), C.nx);
+    s.iy += magic_int(r.y);
+    s.v = m.v;
+    s.o = offset_in(m.pos, magic_value(r));
+    if (RF) {
+        s.clock += inc;
+        s.elapsed = fmaf(dt, k.t_sec, s.elapsed);
+    }
+    load_quad<true, RF>(k, C, s, q);
+    return go;
+}
+
 // Shared-memory pool of particle states for the drain of a case: 9 words per lane
-// (struct of arrays over the block's threads): pid; cx | cy << 16 (grids below 32767
-// cells a side); steps; stop_at | spc << 31; ux, uy, vx, vy, hq.
+// (struct of arrays over the block's threads): pid; ix | iy << 16 (grids below 32767
+// cells a side); steps; stop_at | spc << 31; ox, oy, vx, vy, qm.
 constexpr int POOL_WORDS = 9;
 constexpr int POOL_WORDS_RF = 11;   // + phase, elapsed
 constexpr int TAIL_ROUND_STEPS = 64;
@@ -866,14 +670,15 @@ constexpr int TAIL_ROUND_STEPS = 64;
 template <int RF>
 __device__ __forceinline__ void pool_put(uint32_t *P, int T, int q, const LaneState &s) {
     P[0 * T + q] = (uint32_t)s.pid;
-    P[1 * T + q] = ((uint32_t)s.cx & 0xffffu) | ((uint32_t)s.cy << 16);
+    // a row further below the grid than 16 bits hold stays there: wrapped, it would lead out of the field
+    P[1 * T + q] = ((uint32_t)s.ix & 0xffffu) | ((uint32_t)max(s.iy, -32768) << 16);
     P[2 * T + q] = (uint32_t)s.steps;
     P[3 * T + q] = (uint32_t)s.stop_at | ((uint32_t)s.spc << 31);
-    P[4 * T + q] = __float_as_uint(s.u.x);
-    P[5 * T + q] = __float_as_uint(s.u.y);
+    P[4 * T + q] = __float_as_uint(s.o.x);
+    P[5 * T + q] = __float_as_uint(s.o.y);
     P[6 * T + q] = __float_as_uint(s.v.x);
     P[7 * T + q] = __float_as_uint(s.v.y);
-    P[8 * T + q] = __float_as_uint(s.hq);
+    P[8 * T + q] = __float_as_uint(s.qm);
     if (RF) {
         P[9 * T + q] = s.clock;
         P[10 * T + q] = __float_as_uint(s.elapsed);
@@ -884,17 +689,17 @@ template <int RF>
 __device__ __forceinline__ void pool_get(const uint32_t *P, int T, int q, LaneState &s) {
     s.pid = (int)P[0 * T + q];
     const uint32_t xy = P[1 * T + q];
-    s.cx = (int)(xy & 0xffffu);
-    s.cy = (int)xy >> 16;   // arithmetic shift keeps a negative row
+    s.ix = (int)(xy & 0xffffu);
+    s.iy = (int)xy >> 16;   // arithmetic shift keeps a negative row
     s.steps = (int)P[2 * T + q];
     const uint32_t w = P[3 * T + q];
     s.stop_at = (int)(w & 0x7fffffffu);
     s.spc = (int)(w >> 31);
-    s.u.x = __uint_as_float(P[4 * T + q]);
-    s.u.y = __uint_as_float(P[5 * T + q]);
+    s.o.x = __uint_as_float(P[4 * T + q]);
+    s.o.y = __uint_as_float(P[5 * T + q]);
     s.v.x = __uint_as_float(P[6 * T + q]);
     s.v.y = __uint_as_float(P[7 * T + q]);
-    s.hq = __uint_as_float(P[8 * T + q]);
+    s.qm = __uint_as_float(P[8 * T + q]);
     if (RF) {
         s.clock = P[9 * T + q];
         s.elapsed = __uint_as_float(P[10 * T + q]);
@@ -905,7 +710,7 @@ __device__ __forceinline__ void pool_get(const uint32_t *P, int T, int q, LaneSt
 // needs a decision does not take it and goes inactive), or the first reaches its step cap, or
 // after `limit` steps; particles at their cap end here.  Returns the steps made.  Every lane
 // of the warp calls it.  While every active lane's quad is open the whole warp runs step_open,
-// which has no branch; the cached quad of an inactive lane is marked open.
+// which has no branch.
 template <int RF>
 __device__ __forceinline__ int step_warp(const K32 &k, const CaseView<true> &C, LaneState &s, LaneTally &t,
                                          QuadCache &q, bool &active, int limit, int least) {
@@ -914,14 +719,14 @@ __device__ __forceinline__ int step_warp(const K32 &k, const CaseView<true> &C, 
                                                                            : 0x7fffffffu));
     int j = 0;
     for (;;) {
-        if (C.small_steps && __all_sync(FULL, is_open(q.c00))) {
+        const bool open = !active || (is_open(q.c00) && q.row < C.ny);
+        if (C.small_steps && __all_sync(FULL, open)) {
             step_open<RF>(k, C, s, q, active);
             if (++j >= n) break;
         } else {
             if (!step_near<RF>(k, C, s, q, active) && active) {
                 s.steps += j;
                 active = false;
-                q.mark_open();
             }
             if (++j >= n || __popc(__ballot_sync(FULL, active)) < least) break;
         }
@@ -931,7 +736,6 @@ __device__ __forceinline__ int step_warp(const K32 &k, const CaseView<true> &C, 
         if (s.steps >= s.stop_at) {
             finish_particle<RF>(k, s, t, 3);
             active = false;
-            q.mark_open();
         }
     }
     return j;
@@ -942,26 +746,17 @@ template <int RF>
 __device__ __forceinline__ void step_held(const K32 &k, const CaseView<true> &C, LaneState &s, LaneTally &t,
                                           QuadCache &q, bool &active) {
     if (s.pid >= 0 && !active) {
-        s.cx = min(max(s.cx, 0), C.nx);   // any index after steps that were not finite
-        s.cy = min(s.cy, C.ny);
-        if (s.cy < 0) {                   // below the grid (see LaneState)
-            s.u.y += (float)s.cy;
-            s.cy = 0;
-        }
-        q.base = -1;
-        load_quad<true, RF>(k, C, s, q);
-        ++s.steps;
-        step_decide<RF>(k, C, s, t, q);
+        step_full<true, RF>(k, C, s, t, q);
         active = s.pid >= 0;
-        if (!active) q.mark_open();
+        if (active) load_quad<true, RF>(k, C, s, q);
     }
 }
 
 // Lanes that wait, held for a decision step or empty, before the warp runs the decision
-// steps and the refill for all of them.  Both are long, rarely taken code (about 280
-// instructions) that would otherwise run for one lane at a time; a waiting lane costs a
-// thirty-second of the warp.  2, 3, 4, 6 lanes: 1549, 1473, 1441, 1426 us a batch (AR-8, 2^20
-// particles), 4240, 3974, 3847, 3758 us (2^22 particles, untapered).
+// steps and the refill for all of them.  Both are long, rarely taken code that would otherwise
+// run for one lane at a time; a waiting lane costs a thirty-second of the warp.  4, 6, 8, 10, 14
+// lanes: 1707, 1674, 1674, 1699, 1755 us a batch (60 x 250 cells, 2^20 particles), 4248, 4172, 4177,
+// 4206, 4317 us (2^22 particles, untapered).
 constexpr int WAIT_LANES = 6;
 
 // Traces particles of one case with the calling block until the case's queue is
@@ -996,12 +791,14 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
     C.barrier = a.d_phi != nullptr;
     C.tapered = a.tapered != 0;
     C.first_face = C.barrier || C.tapered;
-    C.small_steps = a.cfl <= 0.45;
+    // a move is at most cfl cells, and 0.02 more where FP32 squares vanish: v^2 and a^2 below 1e-38
+    // count as zero in a step length whose denominator is then 1 m/s alone (1e-9 vscale or more)
+    C.small_steps = a.cfl <= 0.45 && k.inv_v >= 1e-9f;
 
     LaneState s;
     s.pid = -1;
-    s.cx = s.cy = s.steps = s.stop_at = s.spc = 0;
-    s.u.x = s.u.y = s.v.x = s.v.y = s.hq = 0.f;
+    s.ix = s.iy = s.steps = s.stop_at = s.spc = 0;
+    s.o.x = s.o.y = s.v.x = s.v.y = s.qm = 0.f;
     s.clock = 0u;
     s.elapsed = 0.f;
     LaneTally t = {0u, 0u, 0u, 0u, 0u, 0u};
@@ -1009,8 +806,7 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
     q.base = -1;
     q.c00 = q.c01 = q.c10 = q.c11 = tb_fcell{0.f, 0.f};
     q.b00 = q.b01 = q.b10 = q.b11 = make_float4(0.f, 0.f, 0.f, 0.f);
-    q.template load<SMEM, RF>(C.F, k.rf_field, 0, C.P, C.last);
-    q.mark_open();
+    load_quad<SMEM, RF>(k, C, s, q);
     bool active = false;   // the lane holds a particle that is not waiting for a decision step
     bool open = true;
     // The warp's reserved block of claim ranks [wc, we): empty lanes are refilled from it
@@ -1074,11 +870,11 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
                         // converted by the scatter with the expressions below
                         const uint4 r0 = __ldg(k.rec + 2 * rank), r1 = __ldg(k.rec + 2 * rank + 1);
                         s.pid = (int)r0.x;
-                        s.cx = (int)(r0.y & 0xffffu);
-                        s.cy = (int)r0.y >> 16;   // arithmetic: a row below the grid is negative
-                        s.u = make_float2(__uint_as_float(r0.z), __uint_as_float(r0.w));
+                        s.ix = (int)(r0.y & 0xffffu);
+                        s.iy = (int)r0.y >> 16;  // arithmetic shift keeps a negative row
+                        s.o = make_float2(__uint_as_float(r0.z), __uint_as_float(r0.w));
                         s.v = make_float2(__uint_as_float(r1.x), __uint_as_float(r1.y));
-                        s.hq = __uint_as_float(r1.z);
+                        s.qm = __uint_as_float(r1.z);
                         s.spc = (int)(r1.w >> 31);
                         s.steps = (int)(r1.w & 0x7fffffffu);
                         s.stop_at = min(a.max_steps, s.steps + a.step_budget);
@@ -1089,10 +885,10 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
                     if (!REC && idx < n_all && a.d_status[idx] == 3 && a.d_steps[idx] < a.max_steps) {
                         const int pid = (int)idx;
                         s.pid = pid;
-                        start_position(a.d_x[pid], a.d_y[pid], k.inv_dx, C.nx, C.ny, !SMEM, &s.cx, &s.cy, &s.u);
+                        start_position(a.d_x[pid], a.d_y[pid], k.inv_dx, C.nx, C.ny, s.ix, s.iy, s.o);
                         s.v.x = (float)(a.d_vx[pid] * k.inv_v64);
                         s.v.y = (float)(a.d_vy[pid] * k.inv_v64);
-                        s.hq = charge_of(a.d_qm[pid], !SMEM);
+                        s.qm = (float)a.d_qm[pid];
                         s.spc = a.d_spc[pid];
                         s.steps = a.d_steps[pid];
                         s.stop_at = min(a.max_steps, s.steps + a.step_budget);
@@ -1105,7 +901,6 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
                         }
                     }
                     active = s.pid >= 0;
-                    q.base = -1;
                     if (SMEM && active) load_quad<SMEM, RF>(k, C, s, q);
                 }
                 wc = nwc;
@@ -1119,10 +914,10 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
         } else if (__all_sync(FULL, s.pid >= 0)) {
             // step all lanes until a particle ends, one vote per step
             do {
-                cell_step<RF>(k, C, s, t, q);
+                step_full<false, RF>(k, C, s, t, q);
             } while (__all_sync(FULL, s.pid >= 0));
         } else if (s.pid >= 0) {
-            cell_step<RF>(k, C, s, t, q);
+            step_full<false, RF>(k, C, s, t, q);
         }
     }
 
@@ -1141,10 +936,7 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
             if (live == 0) break;
             if ((int)threadIdx.x < live) {
                 pool_get<RF>(pool, T, threadIdx.x, s);
-                q.base = -1;
                 if (SMEM) load_quad<SMEM, RF>(k, C, s, q);
-            } else if (SMEM) {
-                q.mark_open();
             }
             active = s.pid >= 0;
             __syncthreads();
@@ -1156,7 +948,7 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
                         left -= step_warp<RF>(k, C, s, t, q, active, left, __popc(__ballot_sync(FULL, active)));
                         step_held<RF>(k, C, s, t, q, active);
                     } else {
-                        if (s.pid >= 0) cell_step<RF>(k, C, s, t, q);
+                        if (s.pid >= 0) step_full<false, RF>(k, C, s, t, q);
                         --left;
                     }
                 }
@@ -1254,7 +1046,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
 }
 
 // Packs FP64 fields into the halo-padded FP32 tracer layout; one thread per cell.
-__global__ void pack_fields_kernel(int nx, int ny, bool edges, double scale_e, double scale_phi, const uint8_t *vac,
+__global__ void pack_fields_kernel(int nx, int ny, double scale_e, double scale_phi, const uint8_t *vac,
                                    const double *ex, const double *ey, const double *phi,
                                    const double *wface, tb_fcell *out, float4 *bar) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1262,7 +1054,7 @@ __global__ void pack_fields_kernel(int nx, int ny, bool edges, double scale_e, d
     if (c >= cells) return;
     const int ix = c / ny, iy = c - ix * ny;
     const int v = vac[c] ? 1 : 0;
-    tb_store_packed(out, vac, nx, ny, ix, iy, edges, tb_pack_cell(ex[c], ey[c], v, scale_e));
+    tb_store_packed(out, vac, nx, ny, ix, iy, tb_pack_cell(ex[c], ey[c], v, scale_e));
     float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
     if (!v && phi != nullptr) {
         const int w = (ix == 0 ? nx - 1 : ix - 1) * ny + iy;
@@ -1343,7 +1135,7 @@ int tb_launch_pack_fields(tb_ctx *ctx, const double *ex, const double *ey, const
     const double scale_phi = 1.0 / (vscale * vscale);
     const int threads = 256;
     pack_fields_kernel<<<(cells + threads - 1) / threads, threads, 0, s>>>(
-        ctx->nx, ctx->ny, tb_closed_edges(ctx), scale_e, scale_phi, ctx->d_vac, ex, ey, phi, wface, ctx->d_field, ctx->d_barrier);
+        ctx->nx, ctx->ny, scale_e, scale_phi, ctx->d_vac, ex, ey, phi, wface, ctx->d_field, ctx->d_barrier);
     TB_CUDA(ctx, cudaGetLastError());
     ctx->vscale = vscale;
     ctx->fields_ready = 1;
@@ -1397,7 +1189,6 @@ K32 make_k32(const tb_ctx *ctx, const tb_trace_args *a) {
     k.bytes = tb_halo_count(ctx->nx, ctx->ny) * (int)sizeof(tb_fcell);
     k.pool_off = -1;
     k.reverse = ctx->tune_reverse == 1;
-    k.cell_frame = k.bytes > ctx->smem_attr_bytes;
     k.rec = nullptr;
     k.n_rec = nullptr;
     k.okey = nullptr;
@@ -1411,6 +1202,7 @@ K32 make_k32(const tb_ctx *ctx, const tb_trace_args *a) {
     k.t_clock = k.t_sec = k.dt_max = k.bvs = k.bvm = 0.f;
     k.short_steps = false;
     k.wave_scale = 0.f;
+    k.minus_zero = -0.f;
     if (a->n_phase > 0) {
         // step time unit dx / vscale: in seconds, in clock units, and the in-flight step bound
         const double unit = ctx->dx / ctx->vscale;
@@ -1587,14 +1379,14 @@ __device__ __forceinline__ void claim_scatter_body(const K32 &k, int b, int nb) 
             const int32_t n_steps = a.d_steps[i];
             const int8_t sp = a.d_spc[i];
             c = claim_class(kk, ion_class);
-            int cx, cy;
-            float2 u;
-            start_position(x, y, k.inv_dx, k.nx, k.ny, k.cell_frame, &cx, &cy, &u);
+            int ix, iy;
+            float2 o;
+            start_position(x, y, k.inv_dx, k.nx, k.ny, ix, iy, o);
             const float vx = (float)(vx64 * k.inv_v64), vy = (float)(vy64 * k.inv_v64);
-            const float hq = charge_of(qm64, k.cell_frame);
-            r0 = make_uint4((unsigned)i, ((unsigned)cx & 0xffffu) | ((unsigned)cy << 16), __float_as_uint(u.x),
-                            __float_as_uint(u.y));
-            r1 = make_uint4(__float_as_uint(vx), __float_as_uint(vy), __float_as_uint(hq),
+            const float qm = (float)qm64;
+            r0 = make_uint4((unsigned)i, ((unsigned)ix & 0xffffu) | ((unsigned)max(iy, -32768) << 16), __float_as_uint(o.x),
+                            __float_as_uint(o.y));
+            r1 = make_uint4(__float_as_uint(vx), __float_as_uint(vy), __float_as_uint(qm),
                             (unsigned)n_steps | (sp ? 0x80000000u : 0u));
         }
         const unsigned peers = __match_any_sync(0xffffffffu, c);
@@ -1777,7 +1569,7 @@ int tb_launch_trace_f32(tb_ctx *ctx, const tb_trace_args *a, cudaStream_t s) {
         const long long per_sm_n = (a->n + ctx->num_sms - 1) / std::max(ctx->num_sms, 1);
         threads = per_sm_n >= 768 ? 1024 : per_sm_n >= 384 ? 512 : per_sm_n >= 192 ? 256 : 128;
         // circuit_rf with the field in shared memory: at most 512 threads, whose registers hold
-        // the basis fields of a quad.  60 x 250 cells, us a batch at 128, 256, 512 and 1024
+        // the basis fields of a quad (RF_QUAD).  60 x 250 cells, us a batch at 128, 256, 512 and 1024
         // threads: 734, 765, 809, 1093 (405 particles per SM), 925, 844, 901, 1077 (811), 1492, 1030,
         // 1037, 1238 (1771), 2684, 1695, 1253, 1839 (3542), 5131, 3021, 2072, 3393 (7085).
         if (rf && smem) threads = per_sm_n >= 1536 ? 512 : per_sm_n >= 512 ? 256 : 128;
