@@ -1,0 +1,70 @@
+"""What tb_poisson_solve promises beyond its tolerance, at the C entry: the smoother's full division."""
+import ctypes
+import math
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def four_squares(r):
+    a = math.isqrt(r)
+    while True:
+        b = math.isqrt(r - a * a)
+        while b >= 0 and r - a * a - b * b < 1 << 20:
+            rest = r - a * a - b * b
+            for c in range(math.isqrt(rest) + 1):
+                d = math.isqrt(rest - c * c)
+                if c * c + d * d == rest:
+                    return a, b, c, d
+            b -= 1
+        a -= 1
+
+
+def setup(shape, diag, ke, kn, max_rhs):
+    from trench_b200 import _capi
+    from trench_b200.tracer import Context
+    ctx = Context(np.ones(shape, bool), 0, 1.0)
+    ptr = lambda a: np.ascontiguousarray(a).ctypes.data_as(ctypes.c_void_p)  # noqa: E731
+    arrays = [np.ascontiguousarray(a, dtype=np.float64) for a in (diag, ke, kn)] + [np.zeros(shape, np.uint8)]
+    ctx.check(_capi.lib().tb_poisson_setup(ctx.handle, *(ptr(a) for a in arrays), max_rhs))
+    return ctx
+
+
+def solve(ctx, b, x, rtol=1e-13, max_outer=40, inner=12):
+    """(return code, refinement steps, residual); x is the guess and the solution, on the device."""
+    from trench_b200 import _capi
+    from trench_b200.tracer import _ptr
+    iters, resid = ctypes.c_int(), ctypes.c_double()
+    rc = _capi.lib().tb_poisson_solve(ctx.handle, len(b), _ptr(b), _ptr(x), rtol, max_outer, inner, ctypes.byref(iters),
+                                      ctypes.byref(resid), None)
+    return rc, iters.value, resid.value
+
+
+# whole solve in one launch (one and two sides to a cluster); all levels in one CTA; odd widths
+@pytest.mark.parametrize("shape", [(60, 100), (21, 33), (4, 90)])
+@pytest.mark.parametrize("rhs", [1, 20])
+def test_the_smoother_divides_in_full(cuda_device, shape, rhs):
+    """Without couplings one smoothing step is b / d.  With b = +-d, |b| a power of two and so every
+    scaled number exact, one PCG iteration gives +-1 to the last bit, if and only if the FP32
+    quotients are correctly rounded."""
+    import torch
+    rng = np.random.default_rng(shape[0])
+    n = shape[0] * shape[1]
+    d = 2.0 * rng.integers(1, 2048, n) + 1
+    want = rng.choice([-1.0, 1.0], n)
+    d[-4:] = 1.0
+    s = int((d[:-4] ** 2).sum())
+    m = 1
+    while 4 ** m < s:
+        m += 1
+    want[-4:] = four_squares(4 ** m - s)
+    b = d * want
+    ctx = setup(shape, d.reshape(shape), np.zeros(shape), np.zeros(shape), 20)
+    B = torch.from_numpy(np.tile(b, (rhs, 1))).cuda()
+    X = torch.zeros_like(B)
+    rc, iters, resid = solve(ctx, B, X, max_outer=1, inner=1)
+    assert (rc, iters, resid) == (0, 1, 0.0)
+    np.testing.assert_array_equal(X.cpu().numpy(), np.tile(want, (rhs, 1)))
+    ctx.close()
