@@ -158,10 +158,14 @@ int tb_poisson_schedule(tb_ctx *ctx, int pre, int post, int coarse_sweeps);
 int tb_poisson_levels(const tb_ctx *ctx);
 /* Solve L x = b for nrhs right-hand sides, d_b and d_x (nrhs, nx*ny) FP64; d_x is
  * the initial guess on entry.  b must be zero on fixed cells.  Stops when every
- * relative residual |b - L x| / |b| <= rtol, after at most max_outer FP64
- * refinement steps of `inner` FP32 PCG iterations each.  Grids of up to about 24,000 cells
- * are solved by one launch, where each right-hand side stops at its own convergence, and
- * `stream` is synchronised once; larger ones synchronise it once per refinement step.
+ * relative residual |b - L x| / |b| <= rtol (or is at its own FP64 rounding floor), after at
+ * most max_outer FP64 refinement steps of `inner` FP32 PCG iterations each.  Grids that fit the
+ * shared memory of a cluster of 8 CTAs (at least three levels; the widest CTA's columns, 4
+ * ceil(ceil(nx / 4) / 8) of them, hold at most 3584 cells: 60 x 448, 33 x 448, 9 x 896) are solved by
+ * one launch, where each right-hand side stops by itself -- at once if its guess is within rtol,
+ * else at rtol / 10 or where its residual stops falling -- and `stream` is synchronised once.
+ * Larger grids refine all sides until the last is within rtol and synchronise `stream` once per
+ * refinement step.
  * TB_ERR_CONVERGENCE if rtol is not reached. */
 int tb_poisson_solve(tb_ctx *ctx, int nrhs, const double *d_b, double *d_x, double rtol, int max_outer,
                      int inner, int *iters, double *h_resid, void *stream);

@@ -1,4 +1,5 @@
-"""What tb_poisson_solve promises beyond its tolerance, at the C entry: the smoother's full division."""
+"""What tb_poisson_solve promises beyond its tolerance, at the C entry: the smoother's full division, and
+a guess within the tolerance left as it is."""
 import ctypes
 import math
 
@@ -67,4 +68,30 @@ def test_the_smoother_divides_in_full(cuda_device, shape, rhs):
     rc, iters, resid = solve(ctx, B, X, max_outer=1, inner=1)
     assert (rc, iters, resid) == (0, 1, 0.0)
     np.testing.assert_array_equal(X.cpu().numpy(), np.tile(want, (rhs, 1)))
+    ctx.close()
+
+
+# one launch (one and two sides to a cluster), and a launch per pass
+@pytest.mark.parametrize("shape", [(60, 100), (60, 600)])
+@pytest.mark.parametrize("rhs", [1, 20])
+def test_a_guess_within_the_tolerance_is_kept(cuda_device, shape, rhs):
+    import torch
+    rng = np.random.default_rng(8)
+    ke = np.ones(shape)
+    kn = np.ones(shape)
+    kn[:, -1] = 0.0
+    diag = 4.0 + np.zeros(shape)
+    diag[:, 0] += 1.0
+    diag[:, -1] += 1.0
+    ctx = setup(shape, diag, ke, kn, 20)
+    B = torch.from_numpy(rng.normal(0, 1, (rhs, shape[0] * shape[1]))).cuda()
+    X = torch.zeros_like(B)
+    rc, iters, resid = solve(ctx, B, X, rtol=1e-6)
+    assert rc == 0 and iters >= 1 and resid <= 1e-6
+    guess = X.clone()
+    # twice the residual as the tolerance: within it, though not within a tenth of it
+    rc, iters, again = solve(ctx, B, X, rtol=2 * resid)
+    assert (rc, iters) == (0, 0) and torch.equal(X, guess)
+    rc, iters, again = solve(ctx, B, X, rtol=resid / 2)
+    assert rc == 0 and iters >= 1 and again <= resid / 2
     ctx.close()

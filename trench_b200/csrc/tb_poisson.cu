@@ -292,8 +292,8 @@ __device__ __forceinline__ float coupled(const float4 k, const V *x, const int4 
 __device__ __forceinline__ bool is_free(float d) { return d < FLT_MAX; }
 // s / d rounded to the nearest, 0 on fixed cells (whose d is infinite): the reciprocal with one
 // Newton step, and the quotient corrected by its exact remainder (Markstein, IBM J. Res. Dev. 34,
-// 1990; divisors with every mantissa bit set may be one ulp off).  Straight-line: the general division's range check made a solve 1051 instead of 925 us (60
-// x 250 cells).
+// 1990; divisors with every mantissa bit set may be one ulp off).  Straight-line: the general
+// division's range check made a solve 1051 instead of 925 us (60 x 250 cells).
 __device__ __forceinline__ float relaxed(float s, float d) {
     const float f = is_free(d) ? d : 1.f;
     float y = __fdividef(1.f, f);
@@ -840,8 +840,10 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CL_THREADS, 1)
             }
         }
         cluster_sum<3 * R>(cl, sum, sums, parity);
-        // Refined to a tenth of the tolerance, or to the residual's own rounding floor (see
-        // tb_poisson_solve); once within the tolerance, no further than it still falls.
+        // A guess within the tolerance stays as it is.  Otherwise refined to a tenth of the tolerance
+        // (the launches refine every side as long as the worst needs it, most of them further than
+        // the tolerance), or to the residual's own rounding floor (see tb_poisson_solve); once within
+        // the tolerance, no further than it still falls.
         bool go[R], any = false;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -850,7 +852,7 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CL_THREADS, 1)
             aa[r] = sqrt(sum[3 * r + 2]);
             const double rel = bb[r] > 0 ? nr[r] / bb[r] : nr[r];
             go[r] = count[r] == outer && rhs0 + r < A.nrhs &&
-                    !(rel <= 0.1 * A.rtol || nr[r] <= 32.0 * DBL_EPSILON * aa[r] || outer >= A.max_outer ||
+                    !(rel <= (outer == 0 ? A.rtol : 0.1 * A.rtol) || nr[r] <= 32.0 * DBL_EPSILON * aa[r] || outer >= A.max_outer ||
                       (rel <= A.rtol && rel > 0.5 * last[r]));
             last[r] = rel;
             any = any || go[r];
