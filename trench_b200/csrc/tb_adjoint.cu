@@ -286,9 +286,10 @@ __global__ void __launch_bounds__(ONE_BLOCK) k_rev_feedback(const tb_step_desc d
 // shared memory, and a batch takes two cluster barriers.  Sums over CTAs are added in rank
 // order by every CTA, so all of them hold the same bits and the result does not depend on
 // scheduling.  Larger m keeps one launch per step over the whole GPU: there the product
-// itself (8 m^2 bytes) outweighs the launches.  m = 300, 98 table rows, 32 modes, 50 batches:
-// forward 0.53 ms (10.5 us a batch) against 1.1 ms of kernels in 150 launches, reverse 0.50 ms
-// against 1.5 ms in 250.
+// itself (8 m^2 bytes) outweighs the launches.  A sweep of 50 batches with its copies, 98 table
+// rows, us in one launch and in launches: m = 300, 32 modes: forward 830 and 1491, reverse 805 and
+// 2091; m = 440: 950, 1751, 913, 2695 (the operator's rows no longer fit shared memory); m = 760:
+// 1549, 2008, 1408, 3764; m = 1000: 2185, 2131, 1965, 4688; without modes 2135, 2228, 1577, 1830.
 constexpr int FUSED_CTAS = 8;
 constexpr int FUSED_MAX_M = 1024;
 constexpr int FUSED_THREADS = 1024;
@@ -622,11 +623,11 @@ extern "C" int tb_adjoint_forward(tb_ctx *ctx, const tb_step_desc *d, const tb_a
     if (rc != TB_OK) return rc;
     TB_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t s = (cudaStream_t)stream;
-    if (d->m <= FUSED_MAX_M) {
-        size_t bytes = fwd_bytes(d->m);
-        const int keep = d->d_leak_M && bytes + fused_rows_bytes(d->m) <= (size_t)FUSED_SMEM;
-        if (keep) bytes += fused_rows_bytes(d->m);
-        TB_CUDA(ctx, cudaFuncSetAttribute(k_fwd_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, FUSED_SMEM));
+    TB_CUDA(ctx, cudaFuncSetAttribute(k_fwd_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, FUSED_SMEM));
+    size_t bytes = fwd_bytes(d->m);
+    const int keep = d->d_leak_M && bytes + fused_rows_bytes(d->m) <= (size_t)FUSED_SMEM;
+    if (keep) bytes += fused_rows_bytes(d->m);
+    if (d->m <= FUSED_MAX_M && tb_active_clusters(k_fwd_fused, FUSED_CTAS, FUSED_THREADS, bytes) > 0) {
         k_fwd_fused<<<FUSED_CTAS, FUSED_THREADS, bytes, s>>>(*d, *a, keep);
         TB_CUDA(ctx, cudaGetLastError());
         return TB_OK;
@@ -655,12 +656,13 @@ extern "C" int tb_adjoint_reverse(tb_ctx *ctx, const tb_step_desc *d, const tb_a
     cudaStream_t s = (cudaStream_t)stream;
     const int wpb = 8, blocks = (d->m + wpb - 1) / wpb;
     const int rows = a->n_energy + a->n_angle;
+    TB_CUDA(ctx, cudaFuncSetAttribute(k_rev_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, FUSED_SMEM));
+    size_t bytes = rev_bytes(d->m, a->n_basis, rows, a->n_batches);
+    const int keep = d->d_leak_M && bytes + fused_rows_bytes(d->m) <= (size_t)FUSED_SMEM;
+    if (keep) bytes += fused_rows_bytes(d->m);
     if (d->m <= FUSED_MAX_M && a->n_basis <= FUSED_MAX_BASIS && rows <= FUSED_MAX_ROWS &&
-        a->n_batches <= FUSED_MAX_BATCHES) {
-        size_t bytes = rev_bytes(d->m, a->n_basis, rows, a->n_batches);
-        const int keep = d->d_leak_M && bytes + fused_rows_bytes(d->m) <= (size_t)FUSED_SMEM;
-        if (keep) bytes += fused_rows_bytes(d->m);
-        TB_CUDA(ctx, cudaFuncSetAttribute(k_rev_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, FUSED_SMEM));
+        a->n_batches <= FUSED_MAX_BATCHES &&
+        tb_active_clusters(k_rev_fused, FUSED_CTAS, FUSED_THREADS, bytes) > 0) {
         k_rev_fused<<<FUSED_CTAS, FUSED_THREADS, bytes, s>>>(*d, *a, d_lambda, d_gbottom, d_grad, keep);
         TB_CUDA(ctx, cudaGetLastError());
         return TB_OK;

@@ -155,6 +155,28 @@ int tb_cuda_check(tb_ctx *ctx, cudaError_t e, const char *what);
         if (e_ != cudaSuccess) return tb_cuda_check(ctx, e_, #call); \
     } while (0)
 
+// How many clusters of `ctas` CTAs of a kernel (with its cluster size compiled in) the device runs at
+// a time with `bytes` of dynamic shared memory each; 0 where not one fits, as on a part of a GPU.
+template <typename K>
+int tb_active_clusters(K kernel, int ctas, int threads, size_t bytes) {
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)ctas;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = bytes;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
 // Launchers implemented per translation unit.
 int tb_launch_trace_f64(tb_ctx *ctx, const tb_trace_args *a, cudaStream_t s);
 int tb_launch_trace_f32(tb_ctx *ctx, const tb_trace_args *a, cudaStream_t s);

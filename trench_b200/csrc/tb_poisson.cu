@@ -81,6 +81,7 @@ struct tb_poisson {
     int bottom = -1;                           // first level kept in one CTA's shared memory
     int bottom_bytes = 0;                      // its shared memory
     int cluster_bytes[2] = {0, 0};             // shared memory of the one-launch solve of 1 and 2 sides; 0 = does not fit
+    int clusters = 0;                          // clusters of one side that run at a time
     std::vector<float> cd, cke, ckn;           // the coarsest level
     std::vector<uint8_t> cfx;
     float *d_coarse = nullptr;                 // its sweeps as a matrix, by columns (one-launch solve)
@@ -1332,7 +1333,24 @@ extern "C" int tb_poisson_setup(tb_ctx *ctx, const double *h_diag, const double 
         tb_poisson_free(ps);
         return rc;
     }
+    cudaError_t ae = cudaFuncSetAttribute(k_vcycle_bottom, cudaFuncAttributeMaxDynamicSharedMemorySize, BOTTOM_BYTES);
+    if (ae == cudaSuccess)
+        ae = cudaFuncSetAttribute(k_solve_cluster<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_SMEM);
+    if (ae == cudaSuccess)
+        ae = cudaFuncSetAttribute(k_solve_cluster<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_SMEM);
+    if (ae != cudaSuccess) {
+        tb_poisson_free(ps);
+        return tb_cuda_check(ctx, ae, "cudaFuncSetAttribute");
+    }
     cluster_fit(nx, ny, ps->cluster_bytes);
+    if (ps->cluster_bytes[0] > 0) {
+        // where the device cannot run such a cluster the launches keep their work vectors
+        ps->clusters = tb_active_clusters(k_solve_cluster<1>, CLUSTER, CL_THREADS, ps->cluster_bytes[0]);
+        if (ps->clusters < 1) ps->cluster_bytes[0] = ps->cluster_bytes[1] = 0;
+        else if (ps->cluster_bytes[1] > 0 &&
+                 tb_active_clusters(k_solve_cluster<2>, CLUSTER, CL_THREADS, ps->cluster_bytes[1]) < 1)
+            ps->cluster_bytes[1] = 0;
+    }
     // the one-launch solve keeps its vectors in shared memory
     const size_t sides = ps->cluster_bytes[0] > 0 ? 0 : (size_t)max_rhs;
     int lnx = nx, lny = ny;
@@ -1400,15 +1418,6 @@ extern "C" int tb_poisson_setup(tb_ctx *ctx, const double *h_diag, const double 
             return rc;
         }
     }
-    cudaError_t ae = cudaFuncSetAttribute(k_vcycle_bottom, cudaFuncAttributeMaxDynamicSharedMemorySize, BOTTOM_BYTES);
-    if (ae == cudaSuccess)
-        ae = cudaFuncSetAttribute(k_solve_cluster<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_SMEM);
-    if (ae == cudaSuccess)
-        ae = cudaFuncSetAttribute(k_solve_cluster<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_SMEM);
-    if (ae != cudaSuccess) {
-        tb_poisson_free(ps);
-        return tb_cuda_check(ctx, ae, "cudaFuncSetAttribute");
-    }
     ctx->poisson = ps;
     return TB_OK;
 }
@@ -1472,8 +1481,8 @@ extern "C" int tb_poisson_solve(tb_ctx *ctx, int nrhs, const double *d_b, double
         A.rtol = rtol;
         A.coarse = ps->d_coarse;
         // two right-hand sides to a cluster share its barriers once there are more than clusters
-        // that run at a time (16 of 8 SMs); fewer are quicker one to a cluster
-        if (nrhs > 16 && ps->cluster_bytes[1] > 0)
+        // that run at a time; fewer are quicker one to a cluster
+        if (nrhs > ps->clusters && ps->cluster_bytes[1] > 0)
             k_solve_cluster<2><<<(nrhs + 1) / 2 * CLUSTER, CL_THREADS, ps->cluster_bytes[1], s>>>(A);
         else
             k_solve_cluster<1><<<nrhs * CLUSTER, CL_THREADS, ps->cluster_bytes[0], s>>>(A);
