@@ -156,6 +156,9 @@ int tb_poisson_setup(tb_ctx *ctx, const double *h_diag, const double *h_ke, cons
 int tb_poisson_schedule(tb_ctx *ctx, int pre, int post, int coarse_sweeps);
 /* Number of multigrid levels built by tb_poisson_setup (0 before setup). */
 int tb_poisson_levels(const tb_ctx *ctx);
+/* Device bytes that the set-up holds per right-hand side (max_rhs of them): the work vectors of the
+ * launches, next to nothing where one launch keeps them in shared memory. */
+int64_t tb_poisson_side_bytes(const tb_ctx *ctx);
 /* Solve L x = b for nrhs right-hand sides, d_b and d_x (nrhs, nx*ny) FP64; d_x is
  * the initial guess on entry.  b must be zero on fixed cells.  Stops when every
  * relative residual |b - L x| / |b| <= rtol (or is at its own FP64 rounding floor), after at

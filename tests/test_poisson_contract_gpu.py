@@ -1,5 +1,6 @@
 """What tb_poisson_solve promises beyond its tolerance, at the C entry: the smoother's full division, and
-a guess within the tolerance left as it is."""
+a guess within the tolerance left as it is; and the hierarchy built once where a case's set-up has
+no work vectors to give back."""
 import ctypes
 import math
 
@@ -95,3 +96,24 @@ def test_a_guess_within_the_tolerance_is_kept(cuda_device, shape, rhs):
     rc, iters, again = solve(ctx, B, X, rtol=resid / 2)
     assert rc == 0 and iters >= 1 and again <= resid / 2
     ctx.close()
+
+
+@pytest.mark.parametrize("depth,times", [(160, 1), (500, 2)])
+def test_set_up_builds_the_hierarchy_once(cuda_device, monkeypatch, depth, times):
+    """60 x 250 cells: one launch, no work vectors.  60 x 590 cells with 1100 surface cells: 1.7 GB of
+    them, released by a second, narrow set-up."""
+    from dataclasses import replace
+    from trench_b200.fields import FieldSolver
+    from trench_b200.params import Params
+    from trench_b200.step import ChargingCase
+    built = []
+    setup_once = FieldSolver._setup
+    monkeypatch.setattr(FieldSolver, "_setup", lambda self, k: (built.append(k), setup_once(self, k)))
+    p = replace(Params(), nx=60, trench_w=20, trench_d=depth, floor_t=10, mask_t=20, n_vac=60)
+    c = ChargingCase(p, capacity=16, max_batches=4)
+    assert len(built) == times
+    assert built[0] >= c.m
+    if times == 1:
+        assert c.solver.side_bytes * c.solver.max_rhs < 1 << 20
+    else:
+        assert c.solver.side_bytes > 40 * c.n and c.solver.max_rhs == 64

@@ -136,6 +136,7 @@ SIGNATURES = {
     "tb_reserve_claim_order": (ctypes.c_int, [_vp, ctypes.c_longlong]),
     "tb_poisson_setup": (ctypes.c_int, [_vp, _vp, _vp, _vp, _vp, ctypes.c_int]),
     "tb_poisson_levels": (ctypes.c_int, [_vp]),
+    "tb_poisson_side_bytes": (ctypes.c_int64, [_vp]),
     "tb_poisson_schedule": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, ctypes.c_int]),
     "tb_poisson_solve": (ctypes.c_int, [_vp, ctypes.c_int, _vp, _vp, _dbl, ctypes.c_int, ctypes.c_int,
                                         ctypes.POINTER(ctypes.c_int), ctypes.POINTER(_dbl), _vp]),

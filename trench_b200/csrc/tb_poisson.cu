@@ -1445,6 +1445,17 @@ extern "C" int tb_poisson_levels(const tb_ctx *ctx) {
     return (ctx && ctx->poisson) ? (int)ctx->poisson->lev.size() : 0;
 }
 
+extern "C" int64_t tb_poisson_side_bytes(const tb_ctx *ctx) {
+    if (!ctx || !ctx->poisson) return 0;
+    const tb_poisson *ps = ctx->poisson;
+    long long bytes = 8 * sizeof(double);                       // scal
+    if (ps->cluster_bytes[0] > 0) return bytes;
+    const long long n = ps->lev[0].n;
+    for (const Level &L : ps->lev) bytes += 3LL * L.n * (long long)sizeof(float);
+    bytes += n * (long long)(sizeof(double) + 5 * sizeof(float));   // r64; e, pr, pz, pp, pq
+    return bytes + (n + PT - 1) / PT * PART * (long long)sizeof(double);
+}
+
 extern "C" int tb_poisson_solve(tb_ctx *ctx, int nrhs, const double *d_b, double *d_x, double rtol, int max_outer,
                                 int inner, int *iters, double *h_resid, void *stream) {
     if (!ctx) return TB_ERR_ARG;

@@ -204,9 +204,9 @@ class FieldSolver:
             self.psi = psi
             self.D = float(d[c].sum()) - float(torch.dot(self.w, psi))
 
-    # device bytes per right-hand side and cell: the solver's FP32/FP64 work vectors on
-    # all levels (about 44) plus the FP64 right-hand side, solution and temporaries of
-    # solve_rows (about 48)
+    # device bytes per right-hand side and cell: on grids solved by a launch per pass the solver's
+    # FP32/FP64 work vectors on all levels (about 44), and the FP64 right-hand side, solution and
+    # temporaries of solve_rows (about 48)
     BYTES_PER_RHS_CELL = 96
 
     def _setup(self, max_rhs):
@@ -215,11 +215,12 @@ class FieldSolver:
         self.ctx.check(_capi.lib().tb_poisson_setup(self.ctx.handle, ptr(d), ptr(ke), ptr(kn), ptr(fixed),
                                                     int(max_rhs)))
         self.max_rhs = int(max_rhs)
+        self.side_bytes = int(_capi.lib().tb_poisson_side_bytes(self.ctx.handle))
 
     def resize(self, max_rhs):
-        """Right-hand sides per device solve (work vectors are allocated for that many):
-        many for the setup's block solves, where each launch of a small grid is latency-
-        bound and a wider block needs no more launches, few afterwards to hold less memory."""
+        """Right-hand sides per device solve.  On grids solved by a launch per pass the work vectors are
+        allocated for that many (side_bytes each): many for the set-up's block solves, which take no
+        more launches than a few would, few afterwards to hold less memory."""
         if int(max_rhs) != self.max_rhs:
             self._setup(max_rhs)
             self.set_schedule(*self.schedule_used)

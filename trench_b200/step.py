@@ -121,9 +121,9 @@ class ChargingCase:
             eps = geometry.permittivity(solid, mask, p)
             driven = p.field_mode != "floating"
             self.cond, self.eps = cond, eps
-            # the m surface Green's solves run as one block where memory allows (a small grid's
-            # solve is launch-bound, so a block of 340 costs about what a block of 64 does); the
-            # work vectors are sized for that block from the start
+            # the m surface Green's solves run as one block where memory allows: one launch for all of
+            # them on grids that a cluster holds, no more launches than for a few on larger ones,
+            # whose work vectors are sized for that block from the start
             m_surf = int(geometry.surface_cells(solid).sum())
             wide = max(int(max_rhs), FieldSolver.block_size(m_surf, nx * ny))
             self.solver = solver = FieldSolver(self.ctx, p, eps, cond, driven, max_rhs=wide)
@@ -167,7 +167,7 @@ class ChargingCase:
             self.tuning["poisson_schedule"] = self.solver.schedule_used
             sol = self._build_green(rows, green, np.array(extra))
             self.external = (sol[0] + phi_cond.ravel()).reshape(nx, ny)
-            if solver.max_rhs * self.n * (FieldSolver.BYTES_PER_RHS_CELL // 2) > FieldSolver.KEEP_BYTES:
+            if solver.max_rhs * solver.side_bytes > FieldSolver.KEEP_BYTES:
                 solver.resize(max_rhs)
             # leakage (trench_charging_2d.py:768-803)
             self.leak_M = self.leak_h = None
