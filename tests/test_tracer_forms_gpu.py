@@ -134,3 +134,4 @@ def test_fields_that_are_not_finite_stay_in_the_grid(cuda_device, bad):
     clean = trace(vac, *batch(vac, 4001, 12)[:1], *batch(vac, 4001, 12)[1:], 0.35, True, True, "f32")
     same = (got["status"] == clean["status"]) & (got["hit"] == clean["hit"])
     assert same.mean() > 0.8
+    assert (got["status"][~same] == 3).all() and (got["steps"][~same] == 400).all()
