@@ -706,17 +706,26 @@ __device__ __forceinline__ void pool_get(const uint32_t *P, int T, int q, LaneSt
     }
 }
 
+// Lanes that wait, held for a decision step or empty, before the warp runs the decision
+// steps and the refill for all of them.  Both are long, rarely taken code that would otherwise
+// run for one lane at a time; a waiting lane costs a thirty-second of the warp.  4, 6, 8, 10, 14
+// lanes: 1707, 1674, 1674, 1699, 1755 us a batch (60 x 250 cells, 2^20 particles), 4248, 4172, 4177,
+// 4206, 4317 us (2^22 particles, untapered).
+constexpr int WAIT_LANES = 6;
+// Steps after which it does so for fewer lanes: the warp learns only then that the queue is dry, and the
+// block's drain waits for its last warp.
+constexpr int WAIT_STEPS = 64;
+
 // Steps the warp's active lanes together until fewer than `least` are left (a lane whose step
-// needs a decision does not take it and goes inactive), or the first reaches its step cap, or
-// after `limit` steps; particles at their cap end here.  Returns the steps made.  Every lane
-// of the warp calls it.  While every active lane's quad is open the whole warp runs step_open,
-// which has no branch.
+// needs a decision does not take it and goes inactive) or WAIT_STEPS after the first of them,
+// or the first reaches its step cap, or after `limit` steps; particles at their cap end here.
+// Returns the steps made.  Every lane of the warp calls it.  While every active lane's quad is
+// open the whole warp runs step_open, which has no branch.
 template <int RF>
 __device__ __forceinline__ int step_warp(const K32 &k, const CaseView<true> &C, LaneState &s, LaneTally &t,
                                          QuadCache &q, bool &active, int limit, int least) {
     const unsigned FULL = 0xffffffffu;
-    const int n = (int)min((unsigned)limit, __reduce_min_sync(FULL, active ? (unsigned)(s.stop_at - s.steps)
-                                                                           : 0x7fffffffu));
+    int n = (int)min((unsigned)limit, __reduce_min_sync(FULL, active ? (unsigned)(s.stop_at - s.steps) : 0x7fffffffu));
     int j = 0;
     for (;;) {
         const bool open = !active || (is_open(q.c00) && q.row < C.ny);
@@ -728,7 +737,9 @@ __device__ __forceinline__ int step_warp(const K32 &k, const CaseView<true> &C, 
                 s.steps += j;
                 active = false;
             }
-            if (++j >= n || __popc(__ballot_sync(FULL, active)) < least) break;
+            const int left = __popc(__ballot_sync(FULL, active));
+            if (++j >= n || left < least) break;
+            if (left < 32) n = min(n, j + WAIT_STEPS);
         }
     }
     if (active) {
@@ -751,13 +762,6 @@ __device__ __forceinline__ void step_held(const K32 &k, const CaseView<true> &C,
         if (active) load_quad<true, RF>(k, C, s, q);
     }
 }
-
-// Lanes that wait, held for a decision step or empty, before the warp runs the decision
-// steps and the refill for all of them.  Both are long, rarely taken code that would otherwise
-// run for one lane at a time; a waiting lane costs a thirty-second of the warp.  4, 6, 8, 10, 14
-// lanes: 1707, 1674, 1674, 1699, 1755 us a batch (60 x 250 cells, 2^20 particles), 4248, 4172, 4177,
-// 4206, 4317 us (2^22 particles, untapered).
-constexpr int WAIT_LANES = 6;
 
 // Traces particles of one case with the calling block until the case's queue is
 // drained and every particle has ended, then adds the warps' tallies to the case's
@@ -821,7 +825,7 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
 
     for (;;) {
         const bool closed = !open && wc >= we;
-        if (closed || __popc(__ballot_sync(FULL, SMEM ? !active : s.pid < 0)) >= (SMEM ? WAIT_LANES : 1)) {
+        if (closed || __ballot_sync(FULL, SMEM ? !active : s.pid < 0) != 0u) {
             if constexpr (SMEM) step_held<RF>(k, C, s, t, q, active);
             const unsigned need = __ballot_sync(FULL, s.pid < 0);
             if (closed) {
@@ -909,8 +913,9 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
             }
         }
         if constexpr (SMEM) {
-            step_warp<RF>(k, C, s, t, q, active, 0x7fffffff,
-                          closed ? __popc(__ballot_sync(FULL, active)) : 33 - WAIT_LANES);
+            const int occupied = __popc(__ballot_sync(FULL, active));
+            step_warp<RF>(k, C, s, t, q, active, closed || occupied == 32 ? 0x7fffffff : WAIT_STEPS,
+                          closed ? occupied : 33 - WAIT_LANES);
         } else if (__all_sync(FULL, s.pid >= 0)) {
             // step all lanes until a particle ends, one vote per step
             do {
