@@ -1,5 +1,7 @@
-"""The FP32 tracer's pace where its forms of a step have cost time: particles that wait for others.
-A ratio of launches on the same GPU: a block that waits for one warp before its drain doubles it.
+"""The FP32 tracer's pace where its forms of a step have cost time: particles that wait for others, and
+steps beyond the quad.  Ratios of launches on the same GPU, far from what is asserted: a lane that
+waits for the drain doubles the first, a staircase decision at every diagonal move adds a third to
+the second.
 """
 import ctypes
 
@@ -45,3 +47,20 @@ def test_a_few_ended_particles_hold_no_others_up(cuda_device):
     ended = (make(64).alone()["status"] == 1).mean()
     assert 0.05 < ended < 0.5
     assert two < 1.5 * one
+
+
+def test_steps_beyond_the_quad_keep_pace(cuda_device):
+    """A CFL number just above 0.45, where a step may end beyond its quad, against 0.45, in a tapered
+    trench: 10 % fewer steps, each a little longer."""
+    vac = np.zeros((60, 150), bool)
+    vac[:, 100:] = True
+    for j in range(10, 100):
+        w = 8 + (j - 10) // 12
+        vac[30 - w:30 + w, j] = True
+    parts, ex, ey = batch(vac, 1 << 18, 6)
+
+    def make(cfl):
+        return Trace(vac, parts, ex / 30, ey / 30, cfl=cfl, max_steps=2000)
+
+    quad, beyond = least_time(lambda: make(0.45)), least_time(lambda: make(0.5))
+    assert beyond < 1.5 * quad

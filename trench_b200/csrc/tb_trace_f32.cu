@@ -617,30 +617,20 @@ template <int RF>
 __device__ __forceinline__ bool step_near(const K32 &k, const CaseView<true> &C, LaneState &s, QuadCache &q,
                                           bool active) {
     // no branch: some lane of the warp needs the weight, and an open quad's 1 is selected
-    const bool safe = C.small_steps && is_open(q.c00);
+    const bool safe = is_open(q.c00);
     const float weight = vacuum_weight(q);
     float2 A;
     float dt;
     uint32_t inc;
     step_size<RF>(k, C, s, q, safe ? 1.f : weight, A, dt, inc);
     Move m = move_by(k, s, A, dt);
-    bool go;
-    if (C.small_steps) {
-        // the end cell is a corner of the quad (below the grid both rows are copies of row 0)
-        const bool hx = s.o.x >= 0.5f, hy = s.o.y >= 0.5f;
-        const bool right = m.pos.x >= (hx ? 1.f : 0.f), above = m.pos.y >= (hy ? 1.f : 0.f);
-        const float f = right ? (above ? q.c11.ex : q.c10.ex) : (above ? q.c01.ex : q.c00.ex);
-        const bool diagonal = C.tapered && right == hx && above == hy;   // column and row change
-        go = fabsf(m.S.x) < 0.5f && fabsf(m.S.y) < 0.5f && !(above && q.row >= C.ny) &&
-             (safe || ((__float_as_uint(f) & 1u) && !diagonal));
-    } else {
-        const int dix = (int)floorf(m.pos.x), diy = (int)floorf(m.pos.y);
-        const int nix = wrap_column(s.ix + dix, C.nx), niy = s.iy + diy;
-        go = fabsf(m.S.x) < 1.5f && fabsf(m.S.y) < 1.5f && dix >= -1 && dix <= 1 && niy < C.ny &&
-             !(C.tapered && dix != 0 && diy != 0) &&
-             C.F.vac((nix + 1) * C.P + min(max(niy, -1), C.ny) + 1);
-    }
-    go = go && active;
+    // the end cell is a corner of the quad (below the grid both rows are copies of row 0)
+    const bool hx = s.o.x >= 0.5f, hy = s.o.y >= 0.5f;
+    const bool right = m.pos.x >= (hx ? 1.f : 0.f), above = m.pos.y >= (hy ? 1.f : 0.f);
+    const float f = right ? (above ? q.c11.ex : q.c10.ex) : (above ? q.c01.ex : q.c00.ex);
+    const bool diagonal = C.tapered && right == hx && above == hy;   // column and row change
+    const bool go = active && fabsf(m.S.x) < 0.5f && fabsf(m.S.y) < 0.5f && !(above && q.row >= C.ny) &&
+                    (safe || ((__float_as_uint(f) & 1u) && !diagonal));
     if (!go) {
         m.v = s.v;
         m.pos = s.o;
@@ -655,6 +645,41 @@ __device__ __forceinline__ bool step_near(const K32 &k, const CaseView<true> &C,
     if (RF) {
         s.clock += inc;
         s.elapsed = fmaf(dt, k.t_sec, s.elapsed);
+    }
+    load_quad<true, RF>(k, C, s, q);
+    return go;
+}
+
+// The same for steps that may end beyond the quad, but move less than a cell.  In a tapered trench
+// (TAPERED) the two cells beside a change of column and row must be vacuum too: between vacuum
+// cells there is no staircase corner.  Rows are clipped to the halo, which copies the bottom row.
+template <int RF, bool TAPERED>
+__device__ __forceinline__ bool step_far(const K32 &k, const CaseView<true> &C, LaneState &s, QuadCache &q,
+                                         bool active) {
+    float2 A;
+    float dt;
+    uint32_t inc;
+    step_size<RF>(k, C, s, q, vacuum_weight(q), A, dt, inc);
+    const Move m = move_by(k, s, A, dt);
+    const float2 r = magic_floor(m.pos);
+    const int dix = magic_int(r.x), diy = magic_int(r.y);
+    bool go = active && (unsigned)(dix + 1) < 3u && (unsigned)(diy + 1) < 3u && s.iy + diy < C.ny;
+    const int nix = go ? wrap_next(s.ix + dix, C.nx) : s.ix, niy = go ? s.iy + diy : s.iy;
+    const int c0 = (s.ix + 1) * C.P, nc = (nix + 1) * C.P, r0 = max(s.iy, -1) + 1, nr = max(niy, -1) + 1;
+    go = C.F.vac(nc + nr) && go;
+    if (TAPERED) {
+        const bool x_first = C.F.vac(nc + r0), y_first = C.F.vac(c0 + nr);
+        go = go && ((x_first && y_first) || nc == c0 || nr == r0);
+    }
+    if (go) {
+        s.ix = nix;
+        s.iy = niy;
+        s.v = m.v;
+        s.o = offset_in(m.pos, magic_value(r));
+        if (RF) {
+            s.clock += inc;
+            s.elapsed = fmaf(dt, k.t_sec, s.elapsed);
+        }
     }
     load_quad<true, RF>(k, C, s, q);
     return go;
@@ -719,21 +744,24 @@ constexpr int WAIT_STEPS = 64;
 // Steps the warp's active lanes together until fewer than `least` are left (a lane whose step
 // needs a decision does not take it and goes inactive) or WAIT_STEPS after the first of them,
 // or the first reaches its step cap, or after `limit` steps; particles at their cap end here.
-// Returns the steps made.  Every lane of the warp calls it.  While every active lane's quad is
-// open the whole warp runs step_open, which has no branch.
-template <int RF>
+// Returns the steps made.  Every lane of the warp calls it.  With small steps the whole warp runs
+// step_open, which has no branch, while every active lane's quad is open.
+enum StepForm { SMALL_STEPS, FAR_STEPS, FAR_TAPERED };
+template <int RF, StepForm FORM>
 __device__ __forceinline__ int step_warp(const K32 &k, const CaseView<true> &C, LaneState &s, LaneTally &t,
                                          QuadCache &q, bool &active, int limit, int least) {
     const unsigned FULL = 0xffffffffu;
     int n = (int)min((unsigned)limit, __reduce_min_sync(FULL, active ? (unsigned)(s.stop_at - s.steps) : 0x7fffffffu));
     int j = 0;
     for (;;) {
-        const bool open = !active || (is_open(q.c00) && q.row < C.ny);
-        if (C.small_steps && __all_sync(FULL, open)) {
+        const bool open = FORM == SMALL_STEPS && (!active || (is_open(q.c00) && q.row < C.ny));
+        if (FORM == SMALL_STEPS && __all_sync(FULL, open)) {
             step_open<RF>(k, C, s, q, active);
             if (++j >= n) break;
         } else {
-            if (!step_near<RF>(k, C, s, q, active) && active) {
+            const bool went = FORM == SMALL_STEPS ? step_near<RF>(k, C, s, q, active)
+                                                  : step_far<RF, FORM == FAR_TAPERED>(k, C, s, q, active);
+            if (!went && active) {
                 s.steps += j;
                 active = false;
             }
@@ -750,6 +778,13 @@ __device__ __forceinline__ int step_warp(const K32 &k, const CaseView<true> &C, 
         }
     }
     return j;
+}
+template <int RF>
+__device__ __forceinline__ int step_warp(const K32 &k, const CaseView<true> &C, LaneState &s, LaneTally &t,
+                                         QuadCache &q, bool &active, int limit, int least) {
+    if (C.small_steps) return step_warp<RF, SMALL_STEPS>(k, C, s, t, q, active, limit, least);
+    if (C.tapered) return step_warp<RF, FAR_TAPERED>(k, C, s, t, q, active, limit, least);
+    return step_warp<RF, FAR_STEPS>(k, C, s, t, q, active, limit, least);
 }
 
 // The decision steps of the held lanes (occupied, not active).
