@@ -690,7 +690,7 @@ __device__ __forceinline__ bool step_far(const K32 &k, const CaseView<true> &C, 
 // cells a side); steps; stop_at | spc << 31; ox, oy, vx, vy, qm.
 constexpr int POOL_WORDS = 9;
 constexpr int POOL_WORDS_RF = 11;   // + phase, elapsed
-constexpr int TAIL_ROUND_STEPS = 64;
+constexpr int TAIL_ROUND_STEPS = 256;
 
 template <int RF>
 __device__ __forceinline__ void pool_put(uint32_t *P, int T, int q, const LaneState &s) {
