@@ -167,8 +167,8 @@ int64_t tb_poisson_side_bytes(const tb_ctx *ctx);
  * ceil(ceil(nx / 4) / 8) of them, hold at most 3584 cells: 60 x 448, 33 x 448, 9 x 896) are solved by
  * one launch, where each right-hand side stops by itself -- at once if its guess is within rtol,
  * else at rtol / 10 or where its residual stops falling -- and `stream` is synchronised once.
- * Larger grids refine all sides until the last is within rtol and synchronise `stream` once per
- * refinement step.
+ * Larger grids, and more than 120 sides of fewer than 4500 cells, refine all sides until the last is
+ * within rtol and synchronise `stream` once per refinement step.
  * TB_ERR_CONVERGENCE if rtol is not reached. */
 int tb_poisson_solve(tb_ctx *ctx, int nrhs, const double *d_b, double *d_x, double rtol, int max_outer,
                      int inner, int *iters, double *h_resid, void *stream);

@@ -117,3 +117,26 @@ def test_set_up_builds_the_hierarchy_once(cuda_device, monkeypatch, depth, times
         assert c.solver.side_bytes * c.solver.max_rhs < 1 << 20
     else:
         assert c.solver.side_bytes > 40 * c.n and c.solver.max_rhs == 64
+
+
+def test_many_sides_of_a_small_grid(cuda_device):
+    """300 sides of 840 cells go by launches, 100 by one launch: the same solutions."""
+    import torch
+    shape, rhs = (12, 70), 300
+    rng = np.random.default_rng(3)
+    kn = rng.uniform(0.5, 4.0, shape)
+    kn[:, -1] = 0.0
+    ke = rng.uniform(0.5, 4.0, shape)
+    diag = ke + np.roll(ke, 1, axis=0) + kn + np.pad(kn, ((0, 0), (1, 0)))[:, :-1]
+    diag[:, [0, -1]] += 2.0
+    ctx = setup(shape, diag, ke, kn, rhs)
+    B = torch.from_numpy(rng.normal(0, 1, (rhs, 840))).cuda()
+    X, Y = torch.zeros_like(B), torch.zeros_like(B)
+    rc, iters, resid = solve(ctx, B, X)
+    assert rc == 0 and resid <= 1e-13
+    for s in (0, 100, 200):
+        rc, iters, resid = solve(ctx, B[s:s + 100].contiguous(), Y[s:s + 100])
+        assert rc == 0 and resid <= 1e-13
+    # |x - y| <= |L^-1| (|r_x| + |r_y|); the smallest eigenvalue of this operator is above 0.002
+    assert float((X - Y).norm(dim=1).max()) <= 2e-13 / 0.002 * float(B.norm(dim=1).max())
+    ctx.close()

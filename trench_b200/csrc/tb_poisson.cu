@@ -81,7 +81,6 @@ struct tb_poisson {
     int bottom = -1;                           // first level kept in one CTA's shared memory
     int bottom_bytes = 0;                      // its shared memory
     int cluster_bytes[2] = {0, 0};             // shared memory of the one-launch solve of 1 and 2 sides; 0 = does not fit
-    int clusters = 0;                          // clusters of one side that run at a time
     std::vector<float> cd, cke, ckn;           // the coarsest level
     std::vector<uint8_t> cfx;
     float *d_coarse = nullptr;                 // its sweeps as a matrix, by columns (one-launch solve)
@@ -507,6 +506,11 @@ constexpr int CL_CELLS = 7;             // cells of level 0 a thread owns at mos
 constexpr int CL_COARSEST = 64;         // the coarsest level's sweeps as one matrix of at most this size
 constexpr int CL_MAX_LEVELS = 12;
 constexpr int CL_SMEM = 224 * 1024;
+// More sides than this of a grid of fewer cells than this are quicker in launches, which take all
+// of them in every pass.  us in one launch and in launches, 100, 200 and 300 sides: 12 x 70 cells 2240
+// and 2746, 4165 and 3913, 5565 and 4931; 33 x 120 cells 3720 and 3740, 6101 and 5718, 9556 and
+// 7757; 44 x 120 cells 2872 and 3894, 4663 and 6121, 6543 and 8289.
+constexpr int CL_SIDES = 120, CL_FEW_CELLS = 4500;
 
 struct ClusterSolve {
     const Level *lev;
@@ -1243,6 +1247,11 @@ void cluster_fit(int nx, int ny, int bytes[2]) {
     }
 }
 
+// Whether `sides` right-hand sides of n cells are solved by a launch per pass.
+bool launches_solve(const tb_poisson *ps, int n, int sides) {
+    return ps->cluster_bytes[0] == 0 || (sides > CL_SIDES && n < CL_FEW_CELLS);
+}
+
 // The coarsest level's sweeps of the V-cycle (from x = 0, `sweeps` forward then backward) as a
 // matrix, by columns: x = C b.
 std::vector<float> coarsest_matrix(int nx, int ny, const std::vector<float> &d, const std::vector<float> &ke,
@@ -1345,14 +1354,14 @@ extern "C" int tb_poisson_setup(tb_ctx *ctx, const double *h_diag, const double 
     cluster_fit(nx, ny, ps->cluster_bytes);
     if (ps->cluster_bytes[0] > 0) {
         // where the device cannot run such a cluster the launches keep their work vectors
-        ps->clusters = tb_active_clusters(k_solve_cluster<1>, CLUSTER, CL_THREADS, ps->cluster_bytes[0]);
-        if (ps->clusters < 1) ps->cluster_bytes[0] = ps->cluster_bytes[1] = 0;
+        if (tb_active_clusters(k_solve_cluster<1>, CLUSTER, CL_THREADS, ps->cluster_bytes[0]) < 1)
+            ps->cluster_bytes[0] = ps->cluster_bytes[1] = 0;
         else if (ps->cluster_bytes[1] > 0 &&
                  tb_active_clusters(k_solve_cluster<2>, CLUSTER, CL_THREADS, ps->cluster_bytes[1]) < 1)
             ps->cluster_bytes[1] = 0;
     }
     // the one-launch solve keeps its vectors in shared memory
-    const size_t sides = ps->cluster_bytes[0] > 0 ? 0 : (size_t)max_rhs;
+    const size_t sides = launches_solve(ps, n, max_rhs) ? (size_t)max_rhs : 0;
     int lnx = nx, lny = ny;
     for (;;) {
         Level L;
@@ -1449,8 +1458,8 @@ extern "C" int64_t tb_poisson_side_bytes(const tb_ctx *ctx) {
     if (!ctx || !ctx->poisson) return 0;
     const tb_poisson *ps = ctx->poisson;
     long long bytes = 8 * sizeof(double);                       // scal
-    if (ps->cluster_bytes[0] > 0) return bytes;
     const long long n = ps->lev[0].n;
+    if (!launches_solve(ps, (int)n, ps->max_rhs)) return bytes;
     for (const Level &L : ps->lev) bytes += 3LL * L.n * (long long)sizeof(float);
     bytes += n * (long long)(sizeof(double) + 5 * sizeof(float));   // r64; e, pr, pz, pp, pq
     return bytes + (n + PT - 1) / PT * PART * (long long)sizeof(double);
@@ -1473,7 +1482,7 @@ extern "C" int tb_poisson_solve(tb_ctx *ctx, int nrhs, const double *d_b, double
     std::vector<double> sc((size_t)nrhs * 8);
     int outer = 0;
     double worst = 0;
-    const bool small = ps->cluster_bytes[0] > 0;
+    const bool small = !launches_solve(ps, n, nrhs);
     if (small) {
         ClusterSolve A;
         A.lev = ps->d_lev;
@@ -1491,9 +1500,9 @@ extern "C" int tb_poisson_solve(tb_ctx *ctx, int nrhs, const double *d_b, double
         A.scal = ps->scal;
         A.rtol = rtol;
         A.coarse = ps->d_coarse;
-        // two right-hand sides to a cluster share its barriers once there are more than clusters
-        // that run at a time; fewer are quicker one to a cluster
-        if (nrhs > ps->clusters && ps->cluster_bytes[1] > 0)
+        // two right-hand sides to a cluster share its barriers once there are more than run side by
+        // side, 16 of 8 SMs: 16 sides of 33 x 120 cells take 919 us one to a cluster, 1346 two to one
+        if (nrhs > 16 && ps->cluster_bytes[1] > 0)
             k_solve_cluster<2><<<(nrhs + 1) / 2 * CLUSTER, CL_THREADS, ps->cluster_bytes[1], s>>>(A);
         else
             k_solve_cluster<1><<<nrhs * CLUSTER, CL_THREADS, ps->cluster_bytes[0], s>>>(A);
