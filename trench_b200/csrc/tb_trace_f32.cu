@@ -690,7 +690,7 @@ __device__ __forceinline__ bool step_far(const K32 &k, const CaseView<true> &C, 
 // cells a side); steps; stop_at | spc << 31; ox, oy, vx, vy, qm.
 constexpr int POOL_WORDS = 9;
 constexpr int POOL_WORDS_RF = 11;   // + phase, elapsed
-constexpr int TAIL_ROUND_STEPS = 256;
+constexpr int TAIL_ROUND_STEPS = 256;   // 64, 256, 1024: 644, 615, 629 us (2000 particles), 1180, 1151, 1198 (2^19)
 
 template <int RF>
 __device__ __forceinline__ void pool_put(uint32_t *P, int T, int q, const LaneState &s) {
@@ -1609,10 +1609,11 @@ int tb_launch_trace_f32(tb_ctx *ctx, const tb_trace_args *a, cudaStream_t s) {
         const long long per_sm_n = (a->n + ctx->num_sms - 1) / std::max(ctx->num_sms, 1);
         threads = per_sm_n >= 768 ? 1024 : per_sm_n >= 384 ? 512 : per_sm_n >= 192 ? 256 : 128;
         // circuit_rf with the field in shared memory: at most 512 threads, whose registers hold
-        // the basis fields of a quad (RF_QUAD).  60 x 250 cells, us a batch at 128, 256, 512 and 1024
-        // threads: 734, 765, 809, 1093 (405 particles per SM), 925, 844, 901, 1077 (811), 1492, 1030,
-        // 1037, 1238 (1771), 2684, 1695, 1253, 1839 (3542), 5131, 3021, 2072, 3393 (7085).
-        if (rf && smem) threads = per_sm_n >= 1536 ? 512 : per_sm_n >= 512 ? 256 : 128;
+        // the basis fields of a quad (RF_QUAD).  us a launch at 128, 256, 512 and 1024 threads, 60 x
+        // 250 cells: 541, 533, 603, 991 (203 particles per SM), 650, 563, 604, 985 (405), 1051, 808, 693,
+        // 978 (811), 1679, 1134, 887, 1223 (1771), 5752, 3395, 2293, 3467 (7085); 90 x 140 cells: 397,
+        // 385, 432, 704 (203), 537, 409, 464, 705 (405), 903, 649, 592, 781 (811).
+        if (rf && smem) threads = per_sm_n >= 608 ? 512 : per_sm_n >= 256 ? 256 : 128;
     }
     // the drain pool goes after the field when both fit (without the field it always fits
     // under the default 48 KB)
