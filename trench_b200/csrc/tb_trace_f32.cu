@@ -39,9 +39,9 @@
 // What bounds it: instruction issue with the field in shared memory (without the cached quads also
 // the gathers' bank conflicts), one particle's chain of dependent steps in small batches, the
 // gathers' latency with the field in global memory.  Whole batches, one form of a step and no
-// cached quads -> three forms with them: 60 x 200 cells, 6000 particles 893 -> 689 us; 60 x 250
-// cells, 2^20 particles 1728 -> 1613 us, untapered 2^22 particles 4095 -> 3998 us; 8 uneven cases in
-// one launch 3185 -> 2680 us.
+// cached quads -> three forms with them: 60 x 200 cells, 6000 particles 893 -> 546 us; 60 x 250
+// cells, 2^20 particles 1728 -> 1567 us, untapered 2^22 particles 4095 -> 3917 us; 8 uneven cases in
+// one launch 3190 -> 2560 us; above a CFL number of 0.45, 2^19 particles 1653 -> 1410 us (0.5).
 // The step follows the reference algorithm (trench_charging_2d.py:584-650,
 // trench_trace.cu:92-148): vacuum-weighted bilinear field, CFL step, trapezoid
 // update, periodic x, escape at the top, staircase corner crossing, first-face
@@ -190,7 +190,7 @@ constexpr int RF_STEP = 1, RF_QUAD = 2;
 // of a step, ahead of the loop's vote.
 struct QuadCache {
     int base;
-    int row;                    // padded row of the lower corners, before its clamp at the bottom
+    int row;                    // padded row of the lower corners
     float2 t;                   // the particle's position between the corners, in [0, 1)
     tb_fcell c00, c01, c10, c11;
     float4 b00, b01, b10, b11;  // circuit_rf: the basis fields at the same corners
@@ -201,7 +201,7 @@ struct QuadCache {
     // `last`: the largest base whose four corners lie in the field (circuit_rf: a step of dt_max
     // from rest in a field below FP32's squares, or of one that is not a number, may leave the grid)
     template <bool SMEM, int RF>
-    __device__ __forceinline__ void load(const FieldView<SMEM> &F, const float4 *rf_field, int at, int P, int last) {
+    __device__ __forceinline__ void load(const FieldView<SMEM> &F, uint32_t field, const float4 *rf_field, int at, int P, int last) {
         const int b = SMEM && RF ? (int)min((unsigned)at, (unsigned)last) : at;
         if (RF == RF_QUAD && SMEM) {
             asm volatile(
@@ -218,7 +218,7 @@ struct QuadCache {
         }
         if (SMEM) {
             // predicated in place: a branch around the loads costs more than the loads
-            const uint32_t a0 = F.shared_address() + 8u * (unsigned)b, a1 = a0 + 8u * (unsigned)P;
+            const uint32_t a0 = field + 8u * (unsigned)b, a1 = a0 + 8u * (unsigned)P;
             asm volatile(
                 "{\n\t.reg .pred c;\n\t"
                 "setp.ne.s32 c, %8, %9;\n\t"
@@ -247,12 +247,16 @@ struct LaneTally {
 // The quad flag of a quad's lower-left corner (tb_quad_vacuum): all four cells vacuum.
 __device__ __forceinline__ bool is_open(const tb_fcell &c00) { return __float_as_uint(c00.ey) & 1u; }
 
-// Loop-invariant parameters of one case.
-template <bool SMEM>
+// Loop-invariant parameters of one case.  BIASED: quad rows and indexes carry MAGIC_BITS (see
+// load_quad).
+template <bool SMEM_, bool BIASED_>
 struct CaseView {
-    FieldView<SMEM> F;
+    static constexpr bool SMEM = SMEM_, BIASED = BIASED_;
+    FieldView<SMEM_> F;
     int nx, ny, cells, P;
     int last;           // largest quad index
+    int top;            // quad row of the top edge
+    uint32_t field;     // shared-memory address of quad index 0
     float inv_v, cfl;
     bool barrier, tapered, first_face;
     bool small_steps;   // a step moves under half a cell: it ends in a corner cell of its start quad
@@ -286,23 +290,33 @@ __device__ __forceinline__ float2 minus2(float2 a, float2 b) { return __ffma2_rn
 
 // The quad of a particle, the corners (ix - 1 + hx, iy - 1 + hy) .. + 1 where h says whether the
 // offset is in the cell's upper half (in the halo-padded field this needs no wrap, and the
-// clipped rows one clamp), and its position between them, o + 1/2 - h.
-template <bool SMEM, int RF>
-__device__ __forceinline__ void load_quad(const K32 &k, const CaseView<SMEM> &C, const LaneState &s, QuadCache &q) {
-    int col;
-    if (SMEM) {
+// clipped rows one clamp), and its position between them, o + 1/2 - h.  BIASED: h is added with the
+// bits that hold it, MAGIC_BITS too many, which the view's top row and field address allow for:
+// three instructions fewer, 6000 particles 627 -> 546 us a batch, 2^20 1588 -> 1567 us.  Not in
+// case packs, whose kernel has no registers to spare (8 cases 2554 -> 2630 us).
+template <int RF, class View>
+__device__ __forceinline__ void load_quad(const K32 &k, const View &C, const LaneState &s, QuadCache &q) {
+    int col, row;
+    if (View::SMEM) {
         const float2 r = __fadd2_rn(s.o, make_float2(MAGIC, MAGIC));
         q.t = __fadd2_rn(minus2(s.o, magic_value(r)), make_float2(0.5f, 0.5f));
-        col = s.ix + magic_int(r.x);
-        q.row = s.iy + magic_int(r.y);
+        if (View::BIASED) {
+            col = s.ix + __float_as_int(r.x);
+            q.row = row = __viaddmax_s32(s.iy, __float_as_int(r.y), MAGIC_BITS);
+        } else {
+            col = s.ix + magic_int(r.x);
+            q.row = s.iy + magic_int(r.y);
+            row = max(q.row, 0);
+        }
     } else {
         // fewer operations in a row, for steps that wait for the loads
         const bool hx = s.o.x >= 0.5f, hy = s.o.y >= 0.5f;
         q.t = __fadd2_rn(s.o, make_float2(hx ? -0.5f : 0.5f, hy ? -0.5f : 0.5f));
         col = s.ix + hx;
         q.row = s.iy + hy;
+        row = max(q.row, 0);
     }
-    q.template load<SMEM, RF>(C.F, k.rf_field, col * C.P + max(q.row, 0), C.P, C.last);
+    q.template load<View::SMEM, RF>(C.F, C.field, k.rf_field, col * C.P + row, C.P, C.last);
 }
 
 // 1 / (sum of the vacuum corners' weights): solid corners are left out of the field's average.
@@ -325,8 +339,8 @@ __device__ __forceinline__ int rf_interval(const K32 &k, uint32_t clock, float &
 // Acceleration A, time step and (circuit_rf) clock advance of a particle's next step
 // (trench_charging_2d.py:492-509, 587-608): vacuum-weighted bilinear field, with inv_sw =
 // vacuum_weight (1 in an open quad), and the CFL step dt = cfl / (|v| + sqrt(2 |a|) + 1 m/s).
-template <int RF, bool SMEM>
-__device__ __forceinline__ void step_size(const K32 &k, const CaseView<SMEM> &C, const LaneState &s,
+template <int RF, class View>
+__device__ __forceinline__ void step_size(const K32 &k, const View &C, const LaneState &s,
                                           QuadCache &q, float inv_sw, float2 &A, float &dt, uint32_t &inc) {
     const float tx = q.t.x, ty = q.t.y;
     const float2 M1 = make_float2(-1.f, -1.f), txx = make_float2(tx, tx), tyy = make_float2(ty, ty);
@@ -354,7 +368,7 @@ __device__ __forceinline__ void step_size(const K32 &k, const CaseView<SMEM> &C,
         float w0;
         const int i0 = rf_interval(k, c0, w0);
         const float4 e0 = __ldg(k.rf_wave + i0);
-        if (RF == RF_STEP && SMEM) q.load_basis(k.rf_field, C.P);
+        if (RF == RF_STEP && View::SMEM) q.load_basis(k.rf_field, C.P);
         const float4 b00 = q.b00, b01 = q.b01, b10 = q.b10, b11 = q.b11;
         const float ux = __fsub_rn(1.f, tx), uy = __fsub_rn(1.f, ty);
         const float w00 = __fmul_rn(ux, uy), w10 = __fmul_rn(tx, uy), w01 = __fmul_rn(ux, ty), w11 = __fmul_rn(tx, ty);
@@ -451,12 +465,12 @@ __device__ __forceinline__ void finish_particle(const K32 &k, LaneState &s, Lane
 // wall entry, barrier reflection, the step cap; an ended particle's outputs are written and
 // s.pid becomes -1.  Fields in global memory take every step here: those steps wait for the
 // field's loads, and one branch a step costs less than lanes that three forms hold back.
-template <bool SMEM, int RF>
-__device__ __forceinline__ void step_full(const K32 &k, const CaseView<SMEM> &C, LaneState &s, LaneTally &t,
+template <int RF, class View>
+__device__ __forceinline__ void step_full(const K32 &k, const View &C, LaneState &s, LaneTally &t,
                                           QuadCache &q) {
     const tb_trace_args &a = k.a;
     const int nx = C.nx, ny = C.ny, P = C.P;
-    load_quad<SMEM, RF>(k, C, s, q);
+    load_quad<RF>(k, C, s, q);
     // a step below half a cell ends in a corner cell of its quad
     const bool near = !(C.small_steps && is_open(q.c00));
     float2 A;
@@ -467,7 +481,7 @@ __device__ __forceinline__ void step_full(const K32 &k, const CaseView<SMEM> &C,
     // batch); without RF the branch is the better one (200 x 700 cells: 3165 us, 3325 without it)
     float weight = 1.f;
     if (RF) {
-        if (RF == RF_STEP && !SMEM) q.load_basis(k.rf_field, P);
+        if (RF == RF_STEP && !View::SMEM) q.load_basis(k.rf_field, P);
         const float w = vacuum_weight(q);
         weight = near ? w : 1.f;
     } else if (near) {
@@ -488,7 +502,7 @@ __device__ __forceinline__ void step_full(const K32 &k, const CaseView<SMEM> &C,
     const bool escaped = niy >= ny;
     bool hit = false, corner = false;
     if (near && !escaped) {
-        if (!SMEM && C.small_steps && s.iy >= 0) {
+        if (!View::SMEM && C.small_steps && s.iy >= 0) {
             // the end cell is a corner of the quad (saves a load from global memory)
             const bool right = dix >= (s.o.x >= 0.5f ? 1 : 0), above = niy - s.iy >= (s.o.y >= 0.5f ? 1 : 0);
             const float f = right ? (above ? q.c11.ex : q.c10.ex) : (above ? q.c01.ex : q.c00.ex);
@@ -580,8 +594,8 @@ __device__ __forceinline__ void step_full(const K32 &k, const CaseView<SMEM> &C,
 // A step of a warp whose active lanes are all in open quads below the top edge: with small steps
 // it ends in one of the quad's four corner cells, all vacuum and in the grid or below it.  Inactive
 // lanes take a step of length zero, which leaves them exactly as they are.
-template <int RF>
-__device__ __forceinline__ void step_open(const K32 &k, const CaseView<true> &C, LaneState &s, QuadCache &q,
+template <int RF, class View>
+__device__ __forceinline__ void step_open(const K32 &k, const View &C, LaneState &s, QuadCache &q,
                                           bool active) {
     float2 A;
     float dt;
@@ -597,6 +611,12 @@ __device__ __forceinline__ void step_open(const K32 &k, const CaseView<true> &C,
         // (see QuadCache::load: the conversions and the full wrap keep any move's column in the grid)
         s.ix = wrap_column(s.ix + (int)cell.x, C.nx);
         s.iy += (int)cell.y;
+    } else if (View::BIASED) {
+        // a position that is not a number changes neither: one test for both coordinates
+        asm("{\n\t.reg .pred p;\n\tsetp.num.f32 p, %2, %3;\n\t@p add.s32 %0, %0, %4;\n\t@p add.s32 %1, %1, %5;\n\t}"
+            : "+r"(s.ix), "+r"(s.iy)
+            : "f"(m.pos.x), "f"(m.pos.y), "r"(magic_int(r.x)), "r"(magic_int(r.y)));
+        s.ix = wrap_next(s.ix, C.nx);
     } else if (m.pos.x == m.pos.x && m.pos.y == m.pos.y) {
         s.ix = wrap_next(s.ix + magic_int(r.x), C.nx);
         s.iy += magic_int(r.y);
@@ -607,14 +627,14 @@ __device__ __forceinline__ void step_open(const K32 &k, const CaseView<true> &C,
         s.clock += inc;
         s.elapsed = fmaf(dt, k.t_sec, s.elapsed);
     }
-    load_quad<true, RF>(k, C, s, q);
+    load_quad<RF>(k, C, s, q);
 }
 
 // A step of a warp with lanes near a wall or the top edge.  It is taken if it ends in a vacuum
 // cell below the top with no staircase corner on the way; otherwise the particle stays as it was
 // and the return is false: step_full takes that step.
-template <int RF>
-__device__ __forceinline__ bool step_near(const K32 &k, const CaseView<true> &C, LaneState &s, QuadCache &q,
+template <int RF, class View>
+__device__ __forceinline__ bool step_near(const K32 &k, const View &C, LaneState &s, QuadCache &q,
                                           bool active) {
     // no branch: some lane of the warp needs the weight, and an open quad's 1 is selected
     const bool safe = is_open(q.c00);
@@ -629,7 +649,7 @@ __device__ __forceinline__ bool step_near(const K32 &k, const CaseView<true> &C,
     const bool right = m.pos.x >= (hx ? 1.f : 0.f), above = m.pos.y >= (hy ? 1.f : 0.f);
     const float f = right ? (above ? q.c11.ex : q.c10.ex) : (above ? q.c01.ex : q.c00.ex);
     const bool diagonal = C.tapered && right == hx && above == hy;   // column and row change
-    const bool go = active && fabsf(m.S.x) < 0.5f && fabsf(m.S.y) < 0.5f && !(above && q.row >= C.ny) &&
+    const bool go = active && fabsf(m.S.x) < 0.5f && fabsf(m.S.y) < 0.5f && !(above && q.row >= C.top) &&
                     (safe || ((__float_as_uint(f) & 1u) && !diagonal));
     if (!go) {
         m.v = s.v;
@@ -646,15 +666,15 @@ __device__ __forceinline__ bool step_near(const K32 &k, const CaseView<true> &C,
         s.clock += inc;
         s.elapsed = fmaf(dt, k.t_sec, s.elapsed);
     }
-    load_quad<true, RF>(k, C, s, q);
+    load_quad<RF>(k, C, s, q);
     return go;
 }
 
 // The same for steps that may end beyond the quad, but move less than a cell.  In a tapered trench
 // (TAPERED) the two cells beside a change of column and row must be vacuum too: between vacuum
 // cells there is no staircase corner.  Rows are clipped to the halo, which copies the bottom row.
-template <int RF, bool TAPERED>
-__device__ __forceinline__ bool step_far(const K32 &k, const CaseView<true> &C, LaneState &s, QuadCache &q,
+template <int RF, bool TAPERED, class View>
+__device__ __forceinline__ bool step_far(const K32 &k, const View &C, LaneState &s, QuadCache &q,
                                          bool active) {
     float2 A;
     float dt;
@@ -681,7 +701,7 @@ __device__ __forceinline__ bool step_far(const K32 &k, const CaseView<true> &C, 
             s.elapsed = fmaf(dt, k.t_sec, s.elapsed);
         }
     }
-    load_quad<true, RF>(k, C, s, q);
+    load_quad<RF>(k, C, s, q);
     return go;
 }
 
@@ -747,14 +767,14 @@ constexpr int WAIT_STEPS = 64;
 // Returns the steps made.  Every lane of the warp calls it.  With small steps the whole warp runs
 // step_open, which has no branch, while every active lane's quad is open.
 enum StepForm { SMALL_STEPS, FAR_STEPS, FAR_TAPERED };
-template <int RF, StepForm FORM>
-__device__ __forceinline__ int step_warp(const K32 &k, const CaseView<true> &C, LaneState &s, LaneTally &t,
+template <int RF, StepForm FORM, class View>
+__device__ __forceinline__ int step_warp_form(const K32 &k, const View &C, LaneState &s, LaneTally &t,
                                          QuadCache &q, bool &active, int limit, int least) {
     const unsigned FULL = 0xffffffffu;
     int n = (int)min((unsigned)limit, __reduce_min_sync(FULL, active ? (unsigned)(s.stop_at - s.steps) : 0x7fffffffu));
     int j = 0;
     for (;;) {
-        const bool open = FORM == SMALL_STEPS && (!active || (is_open(q.c00) && q.row < C.ny));
+        const bool open = FORM == SMALL_STEPS && (!active || (is_open(q.c00) && q.row < C.top));
         if (FORM == SMALL_STEPS && __all_sync(FULL, open)) {
             step_open<RF>(k, C, s, q, active);
             if (++j >= n) break;
@@ -779,22 +799,22 @@ __device__ __forceinline__ int step_warp(const K32 &k, const CaseView<true> &C, 
     }
     return j;
 }
-template <int RF>
-__device__ __forceinline__ int step_warp(const K32 &k, const CaseView<true> &C, LaneState &s, LaneTally &t,
+template <int RF, class View>
+__device__ __forceinline__ int step_warp(const K32 &k, const View &C, LaneState &s, LaneTally &t,
                                          QuadCache &q, bool &active, int limit, int least) {
-    if (C.small_steps) return step_warp<RF, SMALL_STEPS>(k, C, s, t, q, active, limit, least);
-    if (C.tapered) return step_warp<RF, FAR_TAPERED>(k, C, s, t, q, active, limit, least);
-    return step_warp<RF, FAR_STEPS>(k, C, s, t, q, active, limit, least);
+    if (C.small_steps) return step_warp_form<RF, SMALL_STEPS>(k, C, s, t, q, active, limit, least);
+    if (C.tapered) return step_warp_form<RF, FAR_TAPERED>(k, C, s, t, q, active, limit, least);
+    return step_warp_form<RF, FAR_STEPS>(k, C, s, t, q, active, limit, least);
 }
 
 // The decision steps of the held lanes (occupied, not active).
-template <int RF>
-__device__ __forceinline__ void step_held(const K32 &k, const CaseView<true> &C, LaneState &s, LaneTally &t,
+template <int RF, class View>
+__device__ __forceinline__ void step_held(const K32 &k, const View &C, LaneState &s, LaneTally &t,
                                           QuadCache &q, bool &active) {
     if (s.pid >= 0 && !active) {
-        step_full<true, RF>(k, C, s, t, q);
+        step_full<RF>(k, C, s, t, q);
         active = s.pid >= 0;
-        if (active) load_quad<true, RF>(k, C, s, q);
+        if (active) load_quad<RF>(k, C, s, q);
     }
 }
 
@@ -811,20 +831,26 @@ __device__ __forceinline__ void step_held(const K32 &k, const CaseView<true> &C,
 // rounds: the live particles are packed into the first warps, those warps take up
 // to TAIL_ROUND_STEPS steps, and the rest wait at the barrier.  A particle's
 // arithmetic does not depend on its lane, so the results are the same either way.
-template <bool SMEM, int RF, bool REC = false>
+template <bool SMEM, int RF, bool REC = false, bool PACK = false>
 __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, uint32_t *pool) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const tb_trace_args &a = k.a;
     unsigned long long *const queue = k.queue;
 
-    CaseView<SMEM> C;
+    CaseView<SMEM, SMEM && !RF && !PACK> C;
     C.F.p = fieldp;
     C.nx = k.nx;
     C.ny = k.ny;
     C.cells = k.nx * k.ny;
     C.P = k.ny + 2;  // padded column stride
     C.last = k.nx * C.P + k.ny;
+    C.top = k.ny;
+    C.field = SMEM ? C.F.shared_address() : 0u;
+    if (C.BIASED) {
+        C.top += MAGIC_BITS;
+        C.field -= 8u * ((unsigned)MAGIC_BITS * (unsigned)C.P + (unsigned)MAGIC_BITS);
+    }
     C.inv_v = k.inv_v;
     C.cfl = (float)a.cfl;
     C.barrier = a.d_phi != nullptr;
@@ -845,7 +871,7 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
     q.base = -1;
     q.c00 = q.c01 = q.c10 = q.c11 = tb_fcell{0.f, 0.f};
     q.b00 = q.b01 = q.b10 = q.b11 = make_float4(0.f, 0.f, 0.f, 0.f);
-    load_quad<SMEM, RF>(k, C, s, q);
+    load_quad<RF>(k, C, s, q);
     bool active = false;   // the lane holds a particle that is not waiting for a decision step
     bool open = true;
     // The warp's reserved block of claim ranks [wc, we): empty lanes are refilled from it
@@ -940,7 +966,7 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
                         }
                     }
                     active = s.pid >= 0;
-                    if (SMEM && active) load_quad<SMEM, RF>(k, C, s, q);
+                    if (SMEM && active) load_quad<RF>(k, C, s, q);
                 }
                 wc = nwc;
                 we = nwe;
@@ -954,10 +980,10 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
         } else if (__all_sync(FULL, s.pid >= 0)) {
             // step all lanes until a particle ends, one vote per step
             do {
-                step_full<false, RF>(k, C, s, t, q);
+                step_full<RF>(k, C, s, t, q);
             } while (__all_sync(FULL, s.pid >= 0));
         } else if (s.pid >= 0) {
-            step_full<false, RF>(k, C, s, t, q);
+            step_full<RF>(k, C, s, t, q);
         }
     }
 
@@ -976,7 +1002,7 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
             if (live == 0) break;
             if ((int)threadIdx.x < live) {
                 pool_get<RF>(pool, T, threadIdx.x, s);
-                if (SMEM) load_quad<SMEM, RF>(k, C, s, q);
+                if (SMEM) load_quad<RF>(k, C, s, q);
             }
             active = s.pid >= 0;
             __syncthreads();
@@ -988,7 +1014,7 @@ __device__ __forceinline__ void run_case(const K32 &k, const tb_fcell *fieldp, u
                         left -= step_warp<RF>(k, C, s, t, q, active, left, __popc(__ballot_sync(FULL, active)));
                         step_held<RF>(k, C, s, t, q, active);
                     } else {
-                        if (s.pid >= 0) step_full<false, RF>(k, C, s, t, q);
+                        if (s.pid >= 0) step_full<RF>(k, C, s, t, q);
                         --left;
                     }
                 }
@@ -1078,9 +1104,9 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
             fieldp = reinterpret_cast<const tb_fcell *>(smem_raw);
         }
         uint32_t *pool = k.pool_off >= 0 ? reinterpret_cast<uint32_t *>(smem_raw + k.pool_off) : nullptr;
-        if (k.a.n_phase > 0) run_case<SMEM, RF_STEP>(k, fieldp, pool);  // block-uniform: one case per CTA
-        else if (SMEM && k.rec) run_case<SMEM, 0, SMEM>(k, fieldp, pool);
-        else run_case<SMEM, 0>(k, fieldp, pool);
+        if (k.a.n_phase > 0) run_case<SMEM, RF_STEP, false, true>(k, fieldp, pool);  // block-uniform: one case per CTA
+        else if (SMEM && k.rec) run_case<SMEM, 0, SMEM, true>(k, fieldp, pool);
+        else run_case<SMEM, 0, false, true>(k, fieldp, pool);
         __syncthreads();  // every warp is done with this case's field
     }
 }
