@@ -586,6 +586,17 @@ size_t rev_bytes(int m, int K, int rows, int batches) {
             2 * (size_t)batches) * sizeof(double);
 }
 
+// Whether the device runs the sweeps' clusters at their largest; asked once per context.
+int ask_clusters(tb_ctx *ctx) {
+    if (ctx->adjoint_clusters >= 0) return TB_OK;
+    TB_CUDA(ctx, cudaFuncSetAttribute(k_fwd_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, FUSED_SMEM));
+    TB_CUDA(ctx, cudaFuncSetAttribute(k_rev_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, FUSED_SMEM));
+    const int f = tb_active_clusters(k_fwd_fused, FUSED_CTAS, FUSED_THREADS, FUSED_SMEM);
+    const int r = tb_active_clusters(k_rev_fused, FUSED_CTAS, FUSED_THREADS, FUSED_SMEM);
+    ctx->adjoint_clusters = f < r ? f : r;
+    return TB_OK;
+}
+
 int check_step(tb_ctx *ctx, const tb_step_desc *d, const tb_adjoint_args *a, const char *who) {
     if (d->m < 1 || !d->d_sflag || !d->d_rho_prev || !d->d_work || !(d->dx > 0))
         return tb_fail(ctx, TB_ERR_ARG, "%s: incomplete step descriptor", who);
@@ -623,11 +634,11 @@ extern "C" int tb_adjoint_forward(tb_ctx *ctx, const tb_step_desc *d, const tb_a
     if (rc != TB_OK) return rc;
     TB_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t s = (cudaStream_t)stream;
-    TB_CUDA(ctx, cudaFuncSetAttribute(k_fwd_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, FUSED_SMEM));
+    if ((rc = ask_clusters(ctx)) != TB_OK) return rc;
     size_t bytes = fwd_bytes(d->m);
     const int keep = d->d_leak_M && bytes + fused_rows_bytes(d->m) <= (size_t)FUSED_SMEM;
     if (keep) bytes += fused_rows_bytes(d->m);
-    if (d->m <= FUSED_MAX_M && tb_active_clusters(k_fwd_fused, FUSED_CTAS, FUSED_THREADS, bytes) > 0) {
+    if (d->m <= FUSED_MAX_M && ctx->adjoint_clusters > 0) {
         k_fwd_fused<<<FUSED_CTAS, FUSED_THREADS, bytes, s>>>(*d, *a, keep);
         TB_CUDA(ctx, cudaGetLastError());
         return TB_OK;
@@ -656,13 +667,12 @@ extern "C" int tb_adjoint_reverse(tb_ctx *ctx, const tb_step_desc *d, const tb_a
     cudaStream_t s = (cudaStream_t)stream;
     const int wpb = 8, blocks = (d->m + wpb - 1) / wpb;
     const int rows = a->n_energy + a->n_angle;
-    TB_CUDA(ctx, cudaFuncSetAttribute(k_rev_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, FUSED_SMEM));
+    if ((rc = ask_clusters(ctx)) != TB_OK) return rc;
     size_t bytes = rev_bytes(d->m, a->n_basis, rows, a->n_batches);
     const int keep = d->d_leak_M && bytes + fused_rows_bytes(d->m) <= (size_t)FUSED_SMEM;
     if (keep) bytes += fused_rows_bytes(d->m);
     if (d->m <= FUSED_MAX_M && a->n_basis <= FUSED_MAX_BASIS && rows <= FUSED_MAX_ROWS &&
-        a->n_batches <= FUSED_MAX_BATCHES &&
-        tb_active_clusters(k_rev_fused, FUSED_CTAS, FUSED_THREADS, bytes) > 0) {
+        a->n_batches <= FUSED_MAX_BATCHES && ctx->adjoint_clusters > 0) {
         k_rev_fused<<<FUSED_CTAS, FUSED_THREADS, bytes, s>>>(*d, *a, d_lambda, d_gbottom, d_grad, keep);
         TB_CUDA(ctx, cudaGetLastError());
         return TB_OK;

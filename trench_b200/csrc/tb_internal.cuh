@@ -121,6 +121,7 @@ struct tb_ctx {
     int fields_ready = 0;
     int max_smem = 0;                    // opt-in shared memory per block (bytes)
     int smem_attr_bytes = 0;             // dynamic shared memory set on the FP32 tracer
+    int adjoint_clusters = -1;           // clusters of the adjoint sweeps that run at a time, -1 = not asked yet
     int smem_per_sm = 0;                 // shared memory of one SM (bytes)
     int tune_threads = 0;                // FP32 tracer CTA size (tb_set_tuning), 0 = by batch size
     int tune_ctas_per_sm = 1;            // FP32 tracer CTAs per SM
