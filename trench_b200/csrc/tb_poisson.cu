@@ -27,10 +27,10 @@
 //  * The levels whose vectors and operator fit in one CTA's shared memory (the bottom)
 //    run in one CTA per right-hand side with barriers between the passes, the coarsest
 //    level in one warp.
-//  * A grid whose columns fit in the shared memory of a cluster (up to about 24,000 cells)
-//    is solved whole by one launch (k_solve_cluster): FP64 residual, convergence test, PCG
-//    and V-cycles.  Each right-hand side stops at its own convergence, and the host waits
-//    once.
+//  * A grid whose columns fit in the shared memory of a cluster (cluster_fit: a CTA's columns,
+//    4 ceil(ceil(nx / 4) / 8) of them, hold at most 3584 cells) is solved whole by one launch
+//    (k_solve_cluster): FP64 residual, convergence test, PCG and V-cycles.  Each right-hand
+//    side stops at its own convergence, and the host waits once.
 //  * Larger grids keep one launch per pass over all right-hand sides (their passes are
 //    long enough), with the bottom as one launch.
 #include <cooperative_groups.h>
@@ -498,8 +498,8 @@ __global__ void __launch_bounds__(CTA_THREADS) k_vcycle_bottom(const Level *lev,
 // -- with one halo column on each side, which the owner writes through distributed shared
 // memory when it changes its own edge.  Level 2 and below (a sixteenth of the cells) are CTA 0's.
 // A pass is a few cells a thread between two cluster barriers.  60 x 250, one right-hand side:
-// 0.67 ms (36 PCG iterations of 18 us) against 3.6 ms of kernels and 1.4 ms of gaps between
-// 540 launches; 421 right-hand sides, two to a cluster: 16 ms against 24 ms.
+// 0.71 ms (36 PCG iterations of 19 us) against 3.6 ms of kernels and 1.4 ms of gaps between
+// 540 launches; 300 right-hand sides, two to a cluster: 10.6 ms against 15.8 ms.
 constexpr int CLUSTER = 8;
 constexpr int CL_THREADS = 512;
 constexpr int CL_CELLS = 7;             // cells of level 0 a thread owns at most
