@@ -1,7 +1,6 @@
 """The FP32 tracer's pace where its forms of a step have cost time: particles that wait for others, and
 steps beyond the quad.  Ratios of launches on the same GPU, far from what is asserted: a lane that
-waits for the drain doubles the first, a staircase decision at every diagonal move adds a third to
-the second.
+waits for the drain doubles the first, a staircase decision at every diagonal move the second.
 """
 import ctypes
 
@@ -50,8 +49,8 @@ def test_a_few_ended_particles_hold_no_others_up(cuda_device):
 
 
 def test_steps_beyond_the_quad_keep_pace(cuda_device):
-    """A CFL number just above 0.45, where a step may end beyond its quad, against 0.45, in a tapered
-    trench: 10 % fewer steps, each a little longer."""
+    """A CFL number of 0.9, where a step may end beyond its quad, against 0.45, in a tapered trench: half
+    as many steps, each longer."""
     vac = np.zeros((60, 150), bool)
     vac[:, 100:] = True
     for j in range(10, 100):
@@ -62,5 +61,5 @@ def test_steps_beyond_the_quad_keep_pace(cuda_device):
     def make(cfl):
         return Trace(vac, parts, ex / 30, ey / 30, cfl=cfl, max_steps=2000)
 
-    quad, beyond = least_time(lambda: make(0.45)), least_time(lambda: make(0.5))
+    quad, beyond = least_time(lambda: make(0.45)), least_time(lambda: make(0.9))
     assert beyond < 1.5 * quad

@@ -80,9 +80,9 @@ def trace(vac, n, precision, threads, cfl, n_phase=64):
     return out
 
 
-# automatic shape: 128 threads for 4001 particles, 256 for 150,000, 512 for 300,000
+# automatic shape: 128 threads for 4001 particles, 256 for 60,000, 512 for 150,000 and 300,000
 @pytest.mark.parametrize("kind", ["trench", "posts", "one_column"])
-@pytest.mark.parametrize("n,cfl", [(4001, 0.35), (4001, 0.9), (150_000, 0.35), (300_000, 0.35)])
+@pytest.mark.parametrize("n,cfl", [(4001, 0.35), (4001, 0.9), (60_000, 0.35), (150_000, 0.35), (300_000, 0.35)])
 def test_kept_basis_fields_agree(cuda_device, kind, n, cfl):
     vac = mask_of(kind)
     want = trace(vac, n, "f64", 0, cfl)
